@@ -37,6 +37,7 @@ _LOSS = {"ce": (function.LossFunc.CrossEntropyLoss, function.Activation.Softmax)
          "bce": (function.LossFunc.BinaryCrossEntropy, function.Activation.Sigmoid)}
 _OPTIM = {"adam": function.Optimiser.Adam(0.9, 0.999, 1e-8), "sgd": function.Optimiser.SGD(0.0, False),
           "nesterov": function.Optimiser.SGD(0.9, True)}
+_STEP, _ID_STEP, _LOSS_SCALE = 1000, 1000, 512.0   # steps taken before the first pass; tensor ids between blocks; scale of the deltas
 
 
 def _case(kind, dims, batch, dtype, norm, act, loss="mse", optim="adam", lr=1e-4, dropout=0.0, graph=False, **name):
@@ -115,58 +116,71 @@ def _dims(case):
     return [int(d) for d in case["dims"].split("-")]
 
 
-def prepare(case, seed):
-    dims, batch, prec, train = _dims(case), case["batch"], _PREC[case["dtype"]], case["kind"] == "train"
-    ctx = device.GpuContext(16, 0)
-    core.reset_tensor_ids(0)   # ids seed the dropout masks: as in a fresh process
-    gen = torch.Generator(device=ctx.device)
+def _inputs(case, seed):
+    """What a program has in hand, as plain tensors: the parameters and moments of each block, the input and the target."""
+    dims, batch, train = _dims(case), case["batch"], case["kind"] == "train"
+    dev, dtype = torch.device("cuda", 0), core.TORCH_DTYPE[_PREC[case["dtype"]]]
+    gen = torch.Generator(device=dev)
     gen.manual_seed(seed)
-    half = prec != function.Precision.FP32
-    f32 = function.Precision.FP32
 
     def randn(*shape):
-        return torch.randn(shape, generator=gen, device=ctx.device)
+        return torch.randn(shape, generator=gen, device=dev)
 
     def params(w, b, scale):
-        """Parameters with f32 masters and moments of the size of the gradients."""
-        w, b = w.to(core.TORCH_DTYPE[prec]), b.to(core.TORCH_DTYPE[prec])
-        first = lambda t: core.Tensor(randn(*t.shape).mul_(0.1 * scale), f32)
-        second = lambda t: core.Tensor(torch.rand(t.shape, generator=gen, device=ctx.device).add_(0.5).mul_(scale * scale), f32)
+        """w, b and, for training, dv_w, dv_b, dm_w, dm_b of the size of the gradients."""
+        first = lambda t: randn(*t.shape).mul_(0.1 * scale)
+        second = lambda t: torch.rand(t.shape, generator=gen, device=dev).add_(0.5).mul_(scale * scale)
         dv = second if case["optim"] == "adam" else first
-        return mlp.ParamState(core.Tensor(w, prec), core.Tensor(b, prec),
-                              core.Tensor(w.float(), f32) if half else None, core.Tensor(b.float(), f32) if half else None,
-                              dv(w) if train else None, dv(b) if train else None,
-                              first(w) if train else None, first(b) if train else None)
+        w, b = w.to(dtype), b.to(dtype)
+        return [w, b, dv(w), dv(b), first(w), first(b)] if train else [w, b, None, None, None, None]
 
-    layers = []
-    for i, (k, n) in enumerate(zip(dims[:-1], dims[1:])):
-        hidden = i + 2 < len(dims)
+    blocks = []
+    for k, n in zip(dims[:-1], dims[1:]):
         linear = params(randn(k, n).mul_(math.sqrt(1.5 / k)), randn(1, n).mul_(0.05), 0.5 / math.sqrt(batch))
         norm = params(randn(1, n).mul_(0.1).add_(1.0), randn(1, n).mul_(0.05), 0.5 / math.sqrt(batch))
-        config = LayerInitConfig(_NORM[case["norm"]] if hidden else function.Normalisation.Disabled,
-                                 _ACT[case["act"]] if hidden else function.Activation.Identity,
-                                 function.Regularisation.none(), case["dropout"] if hidden else 0.0)
-        layers.append(mlp.DenseBlock.from_tensors(ctx, train, linear, norm, batch, config, prec))
-    net = ffn.FeedForwardNetwork(layers, dims[0])
+        blocks.append((linear, norm))
 
     if case["loss"] in ("ce", "bce", "mse_sigmoid") and case["norm"] == "none":   # pixels
-        x = torch.randint(0, 256, (batch, dims[0]), generator=gen, device=ctx.device).float().div_(255.0)
+        x = torch.randint(0, 256, (batch, dims[0]), generator=gen, device=dev).float().div_(255.0)
     else:
         x = randn(batch, dims[0])
     if case["loss"] == "ce":
-        t = torch.nn.functional.one_hot(torch.randint(0, dims[-1], (batch,), generator=gen, device=ctx.device), dims[-1]).float()
+        t = torch.nn.functional.one_hot(torch.randint(0, dims[-1], (batch,), generator=gen, device=dev), dims[-1]).float()
     elif case["loss"] == "mse":
         t = randn(batch, dims[-1])
     else:
-        t = torch.rand(batch, dims[-1], generator=gen, device=ctx.device)
-    data = [core.Tensor(d.to(core.TORCH_DTYPE[prec]), prec, take_id=False) for d in (x, t)]
+        t = torch.rand(batch, dims[-1], generator=gen, device=dev)
+    return blocks, x.to(dtype), t.to(dtype)
+
+
+def prepare(case, seed):
+    dims, batch, prec, train = _dims(case), case["batch"], _PREC[case["dtype"]], case["kind"] == "train"
+    blocks, x, t = _inputs(case, seed)
+    ctx = device.GpuContext(16, 0)
+    f32 = function.Precision.FP32
+
+    def state(w, b, *moments):
+        params = [core.Tensor(w, prec), core.Tensor(b, prec)]
+        masters = [core.Tensor(p.float(), f32) if prec != f32 else None for p in (w, b)]
+        return mlp.ParamState(*params, *masters, *(core.Tensor(m, f32) if train else None for m in moments))
+
+    layers = []
+    for i, (linear, norm) in enumerate(blocks):
+        hidden = i + 2 < len(dims)
+        core.reset_tensor_ids(_ID_STEP * i)   # a block's first id, its weights', seeds its dropout masks
+        config = LayerInitConfig(_NORM[case["norm"]] if hidden else function.Normalisation.Disabled,
+                                 _ACT[case["act"]] if hidden else function.Activation.Identity,
+                                 function.Regularisation.none(), case["dropout"] if hidden else 0.0)
+        layers.append(mlp.DenseBlock.from_tensors(ctx, train, state(*linear), state(*norm), batch, config, prec))
+    net = ffn.FeedForwardNetwork(layers, dims[0])
+    data = [core.Tensor(d, prec, take_id=False) for d in (x, t)]
 
     if case["dtype"] == "f32tc":
         # three bf16 parts per operand of the largest product
         ctx.reserve(6 * max(batch * k + k * n + batch * n for k, n in zip(dims[:-1], dims[1:])) + (1 << 20))
         ctx.set_f32_tensor_cores(True)
     optims = [_OPTIM[case["optim"]]] * len(layers)
-    return {"ctx": ctx, "net": net, "x": data[0], "t": data[1], "case": case, "step": 1000,
+    return {"ctx": ctx, "net": net, "x": data[0], "t": data[1], "case": case, "step": _STEP,
             "loss": LossConfig(*_LOSS[case["loss"]]), "train": MultiLayerTrainContext(optims, optims, batch, case["lr"])}
 
 
@@ -202,6 +216,130 @@ def run(state):
         if l.get_mask_coeff() > 0:
             of += [l.get_masks()]
         got.append([t.data for t in of])
+    return got
+
+
+def _f32(v):
+    return float(torch.tensor(v, dtype=torch.float32))
+
+
+def _activation(name, x):
+    return {"relu": lambda: x.clamp_min(0.0), "leaky": lambda: torch.where(x > 0, x, _f32(0.1) * x), "tanh": lambda: x.tanh(),
+            "silu": lambda: x * x.sigmoid(), "mish": lambda: x * torch.nn.functional.softplus(x).tanh(),
+            "sigmoid": lambda: x.sigmoid(), "identity": lambda: x}[name]()
+
+
+def _slope(name, x):
+    """Derivative of the activation at its input x."""
+    if name in ("relu", "leaky"):
+        return torch.where(x > 0, 1.0, 0.0 if name == "relu" else _f32(0.1)).double()
+    sg = x.sigmoid()
+    if name == "tanh":
+        return 1.0 - x.tanh() ** 2
+    if name == "silu":
+        return sg * (1.0 + x * (1.0 - sg))
+    if name == "mish":
+        th = torch.nn.functional.softplus(x).tanh()
+        return th + x * sg * (1.0 - th * th)
+    return sg * (1.0 - sg) if name == "sigmoid" else torch.ones_like(x)
+
+
+def _mask(case, block, shape, dev):
+    """Inverted-dropout mask of the step from the integer hash of row, column, step and tensor id."""
+    u = 0xFFFFFFFF
+    h = ((_STEP + 1) * 1103515245 + _ID_STEP * block) & u
+    h = ((h ^ (h >> 16)) * 1103515245) & u
+    row = torch.arange(shape[0], dtype=torch.int64, device=dev)[:, None]
+    col = torch.arange(shape[1], dtype=torch.int64, device=dev)[None, :]
+    s = ((row * 1103515245) & u) ^ ((col * 0x4C957F2D) & u) ^ (((h ^ (h >> 15)) + row * 7) & u)
+    s = ((s ^ (s >> 17)) * 1103515245 + 12345) & u
+    keep = (s ^ (s >> 15)).float() * 2.0 ** -32 >= case["dropout"]
+    return keep.double() / (1.0 - _f32(case["dropout"]))
+
+
+def exact(case, seed):
+    """The same pass in 64 bits, from the same parameters, moments and data, in plain torch."""
+    need = work(case)
+    if need["bytes"] > 5e9:   # 64-bit tensors of the wide networks would not fit beside the pass
+        return None
+    dims, m, train = _dims(case), case["batch"], case["kind"] == "train"
+    blocks, x, t = _inputs(case, seed)
+    blocks = [[[p if p is None else p.double() for p in of] for of in pair] for pair in blocks]
+    x, t = x.double(), t.double()
+    kept = []   # per block: input, centred or raw values before the normalisation, rstd, preact, predrop, mask, out
+    for i, (linear, norm) in enumerate(blocks):
+        w, b, nw, nb = linear[0], linear[1], norm[0], norm[1]
+        hidden = i + 2 < len(dims)
+        kind = case["norm"] if hidden else "none"
+        z = x @ w + (0.0 if kind == "batch" else b)
+        pre, cen, rstd = z, z, None
+        if kind == "rms":
+            rstd = (z.square().mean(1, keepdim=True) + 1e-6).rsqrt()
+            pre = z * rstd * nw
+        elif kind != "none":
+            over = 1 if kind == "layer" else 0
+            cen = z - z.mean(over, keepdim=True)
+            rstd = (cen.square().mean(over, keepdim=True) + 1e-6).rsqrt()
+            pre = cen * rstd * nw + nb
+        drop = _activation(case["act"] if hidden else "identity", pre)
+        mask = _mask(case, i, z.shape, z.device) if train and hidden and case["dropout"] else torch.ones((), dtype=z.dtype, device=z.device)
+        out = drop * mask
+        kept.append((x, z, cen, rstd, pre, drop, mask, out, kind, hidden))
+        x = out
+    if not train:
+        return [[k[7], k[5], k[4]] + ([k[1], k[2]] if k[8] != "none" else []) for k in kept]
+
+    lr, step = _f32(case["lr"]), _STEP + 1
+    b1, b2, eps = (_f32(0.9), _f32(0.999), _f32(1e-8))
+
+    def update(p, v, mo, g):
+        """(parameter, dv, dm) after the optimiser step on the mean gradient g."""
+        if case["optim"] == "adam":
+            mo, v = b1 * mo + (1.0 - b1) * g, b2 * v + (1.0 - b2) * g * g
+            return p - lr * (mo / (1.0 - b1 ** step)) / ((v / (1.0 - b2 ** step)).sqrt() + eps), v, mo
+        mom = b1 if case["optim"] == "nesterov" else 0.0
+        v = mom * v + g
+        return p - lr * (g + mom * v if case["optim"] == "nesterov" else v), v, mo
+
+    got = [None] * len(blocks)
+    back = None   # gradient at the block's output, times the loss scale
+    for i in reversed(range(len(blocks))):
+        (w, b, vw, vb, mw, mb), (nw, nb, vnw, _, mnw, _) = blocks[i]
+        x, z, cen, rstd, pre, drop, mask, out, kind, hidden = kept[i]
+        if back is None:
+            final = {"ce": "softmax", "mse": "identity", "mse_sigmoid": "sigmoid", "bce": "sigmoid"}[case["loss"]]
+            o = out.softmax(1) if final == "softmax" else _activation(final, out)
+            delta = o - t
+            if case["loss"] == "mse_sigmoid":
+                delta = delta * o * (1.0 - o)
+            out = o if final == "softmax" else out
+            dp = delta * _LOSS_SCALE
+        else:
+            delta = back * _slope(case["act"], pre) * mask
+            dp = delta
+        gnw = torch.zeros_like(z)
+        if kind != "none":
+            gnw = delta * cen * rstd
+            over = dims[i + 1] if kind != "batch" else m
+            # the element-wise form this path uses, not the full derivative of the normalisation
+            dp = nw * rstd * (delta - (rstd * cen) ** 2 / over if kind == "rms"
+                              else delta * (1.0 - 1.0 / over - (rstd * cen) ** 2 / over))
+        scale = 1.0 / (_LOSS_SCALE * m)
+        w, vw, mw = update(w, vw, mw, (x.T @ dp) * scale)
+        if kind != "batch":
+            b, vb, mb = update(b, vb, mb, dp.sum(0, keepdim=True) * scale)
+        of = [out, pre, delta, dp, w, b, vw, vb]
+        if case["optim"] == "adam":
+            of += [mw, mb]
+        if not case["dtype"].startswith("f32"):
+            of += [w]
+        if kind != "none":
+            nw, vnw, mnw = update(nw, vnw, mnw, gnw.sum(0, keepdim=True) * scale)
+            of += [nw, vnw, gnw]
+        if hidden and case["dropout"]:
+            of += [mask]
+        got[i] = of
+        back = dp @ w.T
     return got
 
 
