@@ -1,6 +1,7 @@
 // C ABI of the DenseBlock path: context, argument checks and kernel dispatch.
 // The checks restate DenseBlock's own (Felix1G/soklyn src/mlp.rs:492-519, 548-580,
 // 607-642, 674-736, 756-821) so that a binding can forward status codes unchanged.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -40,6 +41,7 @@ struct sk_ctx {
     uint32_t tc_group_n = 8;               // tile columns walked together (SK_TC_GROUP_N at context creation)
     uint32_t handover_min_rows = 0;        // column sums ride in the dX epilogue from this many rows on (SK_HANDOVER_MIN_ROWS at context creation)
     uint32_t reserve_sms = 0;              // SMs the tensor-core GEMMs leave free (for a concurrent exchange kernel)
+    uint32_t cluster_blocks[4] = {0, 0, 0, 0};   // blocks the chip holds at once in clusters of 1, 2, 4, 8 (one block per SM; 0: none)
     bool lean = false;                     // SK_OPTION_LEAN_BACKWARD
     // data-parallel backward
     uint32_t *dp_counters = nullptr;       // one completion counter per (layer, block), zero between launches
@@ -177,19 +179,87 @@ cudaError_t launch_tc_bn(sk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb
     return cudaGetLastError();
 }
 
+// Tile width and cluster split of one product. Cost in microseconds of one B200 (fitted to single launches): waves
+// of K steps, and what a tile's epilogue adds after the last one; a cluster divides both by its size, pays for the
+// exchange of the partial tiles and has to fit the chip in one wave (a cluster lives in one GPC, whose SM count
+// need not be a multiple of its size: a B200 holds 74 clusters of 2, 33 of 4 and 15 of 8; a sixteenth cluster of 8
+// doubled the time of 512 x 1024 x 3072).
+struct TcPlan { uint32_t bn, split; };
+inline TcPlan plan_tc(const sk_ctx *c, uint32_t M, uint32_t N, uint32_t K, bool gated) {
+    const uint32_t sms = tc_sms(c), num_kb = (K + kTcBK - 1) / kTcBK;
+    auto tiles = [&](uint32_t bn) { return (uint64_t)((M + kTcBM - 1) / kTcBM) * ((N + bn - 1) / bn); };
+    auto cost = [&](uint32_t bn) { return ((tiles(bn) + sms - 1) / sms) * bn; };
+    // A 128-wide tile re-reads the A panel twice as often per flop and measured about 0.8 of the
+    // 256-wide tile's rate at equal occupancy, so it has to save more than a fifth of the waves.
+    TcPlan best{N > 128 && cost(256) * 4 <= cost(128) * 5 ? 256u : 128u, 1u};
+    if (gated || tiles(best.bn) >= sms || num_kb > (1u << 26)) return best;
+    double least = 0.0;
+    for (uint32_t bn = 128; bn <= (N > 128 ? 256u : 128u); bn += 128)
+        for (uint32_t split = 1, i = 0; split <= 8 && split <= num_kb; split *= 2, ++i) {
+            if (split > 1 && tiles(bn) * split > std::min(sms, c->cluster_blocks[i])) break;
+            if (split == 1 && bn != best.bn) continue;
+            const double us = ((num_kb + split - 1) / split) * (bn == 256 ? 0.30 : 0.20) + (bn / 128) * 5.0 / split + (split > 1 ? 1.5 : 0.0);
+            if (least == 0.0 || us < least) { least = us; best = TcPlan{bn, split}; }
+        }
+    return best;
+}
+
+// How many blocks of the cluster kernel the chip holds at once, by cluster size.
+void query_cluster_blocks(sk_ctx *c) {
+    auto kernel = gemm_tc_cluster_kernel<false, true, 256, EpiForward<__half>>;
+    constexpr int smem = TcClusterShape<256>::kSmemBytes;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return; }
+    for (uint32_t i = 0, split = 1; i < 4; ++i, split *= 2) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(split * 64);
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); clusters = 0; }
+        c->cluster_blocks[i] = (uint32_t)clusters * split;
+    }
+}
+
+template <typename T, bool A_MN, bool B_MN, int BN, class Epi>
+cudaError_t launch_tc_cluster(sk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb, uint32_t M, uint32_t N, uint32_t K,
+                              const Epi &epi, uint32_t group_n, uint32_t split) {
+    using S = TcClusterShape<BN>;
+    static uint64_t attr_set[4] = {0, 0, 0, 0};   // devices 0..255
+    auto kernel = gemm_tc_cluster_kernel<A_MN, B_MN, BN, Epi>;
+    const unsigned dev = (unsigned)c->device & 255u;
+    if (!(attr_set[dev >> 6] >> (dev & 63) & 1ull)) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmemBytes);
+        if (e != cudaSuccess) return e;
+        attr_set[dev >> 6] |= 1ull << (dev & 63);
+    }
+    const uint32_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + BN - 1) / BN);
+    const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, kTcBM, BN);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(tiles * split);
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = S::kSmemBytes;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    c->tc_launches++;
+    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, M, N, K, idesc, group_n, epi, c->tc_err);
+}
+
 // C[M x N] = A.B on the tensor cores. A_MN / B_MN: operand contiguous along M / N (else along K).
 template <typename T, bool A_MN, bool B_MN, class Epi>
 cudaError_t launch_gemm_tc(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, const T *B, size_t ldb, uint32_t M,
                            uint32_t N, uint32_t K, const Epi &epi, const TcGate &gate = TcGate{}) {
-    const uint32_t sms = tc_sms(c);
-    auto cost = [&](uint32_t bn) {
-        const uint64_t tiles = (uint64_t)((M + kTcBM - 1) / kTcBM) * ((N + bn - 1) / bn);
-        return ((tiles + sms - 1) / sms) * bn;
-    };
-    // A 128-wide tile re-reads the A panel twice as often per flop and measured about 0.8 of the
-    // 256-wide tile's rate at equal occupancy, so it has to save more than a fifth of the waves.
-    const bool wide = N > 128 && cost(256) * 4 <= cost(128) * 5;
-    const uint32_t bn = wide ? 256 : 128;
+    const TcPlan plan = plan_tc(c, M, N, K, gate.flags != nullptr);
+    const bool wide = plan.bn == 256;
+    const uint32_t bn = plan.bn;
     CUtensorMap ta, tb;
     const bool ok_a = A_MN ? get_tmap(c, A, dtype, M, K, lda, 64, &ta) : get_tmap(c, A, dtype, K, M, lda, kTcBM, &ta);
     const bool ok_b = B_MN ? get_tmap(c, B, dtype, N, K, ldb, 64, &tb) : get_tmap(c, B, dtype, K, N, ldb, bn, &tb);
@@ -200,6 +270,9 @@ cudaError_t launch_gemm_tc(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, co
         if (per_chunk >= 1 && per_chunk < group_n) group_n = per_chunk;
         if (per_chunk == 0) group_n = 1;
     }
+    if (plan.split > 1)
+        return wide ? launch_tc_cluster<T, A_MN, B_MN, 256, Epi>(c, ta, tb, M, N, K, epi, group_n, plan.split)
+                    : launch_tc_cluster<T, A_MN, B_MN, 128, Epi>(c, ta, tb, M, N, K, epi, group_n, plan.split);
     return wide ? launch_tc_bn<T, A_MN, B_MN, 256, Epi>(c, ta, tb, M, N, K, epi, gate, group_n)
                 : launch_tc_bn<T, A_MN, B_MN, 128, Epi>(c, ta, tb, M, N, K, epi, gate, group_n);
 }
@@ -455,7 +528,8 @@ int hidden_error_impl(sk_ctx *c, const sk_dense *cur, const sk_dense *next, uint
     const bool specialised = !f32 && ((cur->act == SK_ACT_SILU && cur->norm == SK_NORM_RMS) ||
                                       (cur->act == SK_ACT_MISH && cur->norm == SK_NORM_LAYER));
     if ((c->in_ffn_backward || c->colsum_handover) && specialised && batch >= c->handover_min_rows && epi.vec_ok && tc_eligible(c, cur->dtype, dy, ec, wn, ec)) {
-        const uint32_t groups = (batch + 31) / 32;
+        const uint32_t split = plan_tc(c, batch, cur->N, ec, gate.flags != nullptr).split;
+        const uint32_t groups = split == 1 ? (batch + 31) / 32 : (batch + kTcBM - 1) / kTcBM * split * kTcEpiWarps;
         const size_t need = ((size_t)groups + kColsumFold) * 3 * cur->N * sizeof(float);
         if (need <= c->workspace_bytes) {
             epi.colsum_partial = (float *)c->workspace; epi.colsum_groups = groups;
@@ -879,6 +953,7 @@ int sk_ctx_create(int device, uint32_t tile_dim, void *stream, int create_stream
     cudaFuncSetAttribute(sk::norm_rows_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     cudaFuncSetAttribute(sk::norm_rows_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     c->cc_major = prop.major;
+    if (c->cc_major == 10) query_cluster_blocks(c);
     if (const char *env = getenv("SK_TC_GROUP_N")) { const int v = atoi(env); if (v >= 1 && v <= 64) c->tc_group_n = (uint32_t)v; }
     c->handover_min_rows = kHandoverMinRows;
     if (const char *env = getenv("SK_HANDOVER_MIN_ROWS")) { const int v = atoi(env); if (v >= 32) c->handover_min_rows = (uint32_t)v; }

@@ -162,8 +162,8 @@ template <typename T, int ACT = -1, int NORM = -1> struct EpiHidden {
     uint32_t N, norm, act;
     float leaky, inv_n, inv_m;
     bool vec_ok;
-    // Optional: column sums of d_prenorm, d_norm_w and d_norm_b per group of 32 rows, written as
-    // partial[group][which][col] while the values are in registers, so that the weight-update call
+    // Optional: column sums of d_prenorm, d_norm_w and d_norm_b per group of rows (32 adjacent ones, or those of one warp
+    // of a cluster), written as partial[group][which][col] while the values are in registers, so that the weight-update call
     // that follows need not read the three tensors again. Only with vec_ok and on the tensor-core
     // kernel (every element then goes through finish()).
     float *colsum_partial;
@@ -297,6 +297,25 @@ template <typename T, int ACT = -1, int NORM = -1> struct EpiHidden {
         }
         if (valid && lane < 4 && group < colsum_groups) {
             float *base = colsum_partial + (size_t)group * 3 * N + col0;
+            store_run<float, 8>(base, true, a.dp);
+            store_run<float, 8>(base + N, true, a.gw);
+            store_run<float, 8>(base + 2 * (size_t)N, true, a.gb);
+        }
+    }
+    // Called by all 32 lanes of a warp after all its rows: lanes 16-31 hold the columns of lanes 0-15 (`halves`) or
+    // columns of their own.
+    __device__ __forceinline__ void slab_store(Acc &a, uint32_t slab, uint32_t col0, bool halves, uint32_t lane) const {
+        if (!colsum_partial) return;
+        if (halves) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                a.dp[j] += __shfl_xor_sync(0xffffffffu, a.dp[j], 16);
+                a.gw[j] += __shfl_xor_sync(0xffffffffu, a.gw[j], 16);
+                a.gb[j] += __shfl_xor_sync(0xffffffffu, a.gb[j], 16);
+            }
+        }
+        if (col0 < N && (!halves || lane < 16) && slab < colsum_groups) {
+            float *base = colsum_partial + (size_t)slab * 3 * N + col0;
             store_run<float, 8>(base, true, a.dp);
             store_run<float, 8>(base + N, true, a.gw);
             store_run<float, 8>(base + 2 * (size_t)N, true, a.gb);

@@ -443,4 +443,182 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (warp == 1) tc::tmem_dealloc(tmem_base, kTmemCols);
 }
 
+// ---- few output tiles: one tile per cluster, K split over its blocks ------------------------------------
+// A product with fewer tiles than SMs leaves the persistent kernel's chip idle twice: the K loop of a tile is
+// serial, and so is its epilogue (eight warps work through 128 x BN outputs, a memory round trip per pass).
+// Here the S blocks of a cluster (blockIdx.x / S = tile) each accumulate a contiguous share of the K steps, put
+// their partial tile into their own shared memory (the stage ring is free by then), and after a cluster barrier
+// every block adds up, in rank order, and finishes every S-th group of rows: the partial sums travel through
+// distributed shared memory, not HBM, the order of the sum is fixed, and the epilogue is spread over S times as many
+// SMs. Operands, stages, descriptors and functors are those of gemm_tc_kernel. A row of the partial tile is kept as
+// two planes (the first and the second four columns of every run of 8), so that a warp's remote loads are
+// contiguous: with the two halves of a run side by side, every load touched 8 rows and half of each 32-byte piece,
+// and the exchange of 16 tiles of 128 x 256 over clusters of 8 took 30 us.
+template <int BN> struct TcClusterShape {
+    using S = TcShape<BN>;
+    static constexpr int kPitch = BN + 4;          // floats: rows 4 banks apart, float4 accesses conflict-free both ways
+    static constexpr int kBarBytes = (2 * S::kStages + 1) * 8 + 16;
+    static constexpr int kSmemBytes = 1024 + S::kStages * S::kStageBytes + kBarBytes;
+    static_assert(kTcBM * kPitch * 4 <= S::kStages * S::kStageBytes, "the partial tile fits the stage ring");
+};
+
+template <bool A_MN, bool B_MN, int BN, class Epi>
+__global__ void __launch_bounds__(kTcThreads, 1)
+gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                       uint32_t M, uint32_t N, uint32_t K, uint32_t idesc, uint32_t group_n, Epi epi, int *err_flag) {
+    using S = TcShape<BN>;
+    constexpr int kPitch = TcClusterShape<BN>::kPitch;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *stages = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    float *partial = reinterpret_cast<float *>(stages);
+    uint64_t *full_bar = reinterpret_cast<uint64_t *>(stages + S::kStages * S::kStageBytes);
+    uint64_t *empty_bar = full_bar + S::kStages;
+    uint64_t *tmem_full = empty_bar + S::kStages;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_full + 1);
+    uint32_t *gave_up = tmem_slot + 1;             // a bounded wait of this block ran out: its partial tile is not valid
+
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = tc::cluster_rank(), split = tc::cluster_size();
+    const uint32_t tiles_m = (M + kTcBM - 1) / kTcBM, tiles_n = (N + BN - 1) / BN;
+    const uint32_t num_kb = (K + kTcBK - 1) / kTcBK;
+    const uint32_t kb0 = rank * num_kb / split, kb1 = (rank + 1) * num_kb / split;   // host: split <= num_kb <= 2^26
+    uint32_t mi, ni;
+    tile_coords(blockIdx.x / split, tiles_m, tiles_n, group_n, mi, ni);
+    const uint32_t m0 = mi * kTcBM, n0 = ni * BN;
+
+    if (warp == 0 && lane == 0) {
+        tc::prefetch_tensormap(&tmap_a);
+        tc::prefetch_tensormap(&tmap_b);
+        for (int s = 0; s < S::kStages; ++s) { tc::mbar_init(&full_bar[s], 1); tc::mbar_init(&empty_bar[s], 1); }
+        tc::mbar_init(tmem_full, 1);
+        *gave_up = 0;
+        tc::fence_barrier_init();
+    }
+    if (warp == 1) {
+        tc::tmem_alloc(tmem_slot, BN);
+        tc::tmem_relinquish();
+    }
+    tc::tc_fence_before_sync();
+    __syncthreads();
+    tc::tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t stage = 0, phase = 0;
+            for (uint32_t kb = kb0; kb < kb1; ++kb) {
+                if (!tc::mbar_wait(&empty_bar[stage], phase ^ 1)) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrProducer); break; }
+                tc::mbar_arrive_expect_tx(&full_bar[stage], S::kStageBytes);
+                uint8_t *sa = stages + stage * S::kStageBytes, *sb = sa + kTcABytes;
+                const int32_t k0 = kb * kTcBK;
+                if (A_MN) {
+#pragma unroll
+                    for (int j = 0; j < kTcBM / 64; ++j) tc::tma_load_2d(sa + j * 8192, &tmap_a, &full_bar[stage], m0 + j * 64, k0);
+                } else {
+                    tc::tma_load_2d(sa, &tmap_a, &full_bar[stage], k0, m0);
+                }
+                if (B_MN) {
+#pragma unroll
+                    for (int j = 0; j < BN / 64; ++j) tc::tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[stage], n0 + j * 64, k0);
+                } else {
+                    tc::tma_load_2d(sb, &tmap_b, &full_bar[stage], k0, n0);
+                }
+                if (++stage == S::kStages) { stage = 0; phase ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            uint32_t stage = 0, phase = 0;
+            bool ok = true;
+            for (uint32_t kb = kb0; kb < kb1; ++kb) {
+                if (!tc::mbar_wait(&full_bar[stage], phase)) { ok = false; break; }
+                tc::tc_fence_after_sync();
+                const uint32_t sa = tc::smem_u32(stages + stage * S::kStageBytes), sb = sa + kTcABytes;
+#pragma unroll
+                for (int j = 0; j < kTcBK / 16; ++j) {
+                    const uint64_t da = A_MN ? tc::make_smem_desc(sa + j * 2048, 8192, 1024) : tc::make_smem_desc(sa + j * 32, 16, 1024);
+                    const uint64_t db = B_MN ? tc::make_smem_desc(sb + j * 2048, 8192, 1024) : tc::make_smem_desc(sb + j * 32, 16, 1024);
+                    tc::umma_f16(tmem_base, da, db, idesc, kb > kb0 || j > 0);
+                }
+                tc::umma_commit(&empty_bar[stage]);
+                if (++stage == S::kStages) { stage = 0; phase ^= 1; }
+            }
+            if (!ok) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrMma); }
+            tc::umma_commit(tmem_full);
+        }
+    } else {
+        // the whole accumulator of this block to shared memory, rows that exist only
+        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
+        if (!tc::mbar_wait(tmem_full, 0)) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrEpilogue); }
+        tc::tc_fence_after_sync();
+        if (m0 + quarter * 32 < M) {
+            float *dst = partial + (quarter * 32 + lane) * kPitch;
+#pragma unroll 1
+            for (uint32_t c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
+                if (n0 + c0 >= N) break;
+                float v[32];
+                tc::tmem_ld_32x32(tmem_base + ((quarter * 32) << 16) + c0, v);
+#pragma unroll
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4 *>(dst + (j & 4) / 4 * (BN / 2) + (c0 + j) / 8 * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            }
+        }
+        tc::tc_fence_before_sync();
+    }
+    __syncwarp();
+    tc::cluster_sync();
+
+    // a block whose waits ran out has filled in no valid tile: the cluster then writes nothing
+    bool valid = true;
+    for (uint32_t r = 0; r < split; ++r) valid = valid && tc::ld_cluster_u32(tc::map_shared(tc::smem_u32(gave_up), r)) == 0;
+    if (warp >= 2 && valid) {
+        constexpr uint32_t kLanesRow = BN / 8, kRows = 32 / kLanesRow;      // rows per warp and pass: 1 (BN = 256) or 2
+        const uint32_t units = (min((uint32_t)kTcBM, M - m0) + kRows - 1) / kRows, run = lane % kLanesRow;
+        const uint32_t col = n0 + run * 8, ncols = col < N ? min(8u, N - col) : 0u;
+        const bool fast = epi.vec_ok && ncols == 8;
+        const uint32_t base = tc::smem_u32(partial) + run * 16;
+        typename Epi::Cols cols;
+        if (fast) epi.cols(col, cols);
+        typename EpiAcc<Epi>::type sums;
+        if constexpr (EpiAcc<Epi>::value) epi.acc_init(sums);
+#pragma unroll 1
+        for (uint32_t u = (warp - 2) * split + rank; u < units; u += kTcEpiWarps * split) {
+            const uint32_t row = m0 + u * kRows + lane / kLanesRow;
+            if (row >= M || ncols == 0) continue;
+            typename Epi::Pre pre;
+            if (fast) epi.prefetch(row, col, pre);
+            const uint32_t at = base + (row - m0) * kPitch * 4;
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+            for (uint32_t r = 0; r < split; r += 2) {          // split is a power of two
+                const uint32_t a = tc::map_shared(at, r), b = tc::map_shared(at, r + 1);
+                const float4 a0 = tc::ld_cluster_f4(a), a1 = tc::ld_cluster_f4(a + BN * 2);
+                const float4 b0 = tc::ld_cluster_f4(b), b1 = tc::ld_cluster_f4(b + BN * 2);
+                v[0] += a0.x; v[1] += a0.y; v[2] += a0.z; v[3] += a0.w;
+                v[4] += a1.x; v[5] += a1.y; v[6] += a1.z; v[7] += a1.w;
+                v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
+                v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+            }
+            if (fast) {
+                if constexpr (EpiAcc<Epi>::value) epi.finish(row, col, v, pre, cols, sums);
+                else epi.finish(row, col, v, pre, cols);
+            } else {
+                epi.template run<8>(row, col, v, ncols);
+            }
+        }
+        // running sums: one slab per warp of the cluster, over all its rows of the tile
+        if constexpr (EpiAcc<Epi>::value) {
+            __syncwarp();
+            epi.slab_store(sums, (mi * split + rank) * kTcEpiWarps + warp - 2, col, kRows == 2, lane);
+        }
+    }
+    __syncwarp();
+    tc::cluster_sync();     // no block leaves while another still reads its partial tile
+    if (warp == 1) {
+        tc::tc_fence_after_sync();
+        tc::tmem_dealloc(tmem_base, BN);
+    }
+}
+
 } // namespace sk

@@ -1,0 +1,36 @@
+"""One training step against the CPU oracle at the sizes where the kernel choice changes or a tile, cluster or copy has a
+ragged end. Tolerances as in test_parity_gpu.py: 1e-5 of a tensor's largest value in f32 (5e-5 with the tensor-core
+option: its products are within 2e-6 element by element, the norm backward amplifies them), 1e-2 in 16 bits, whose
+storage rounds every tensor of the chain to 2^-12 in f16. bf16 rounds to 2^-9: the two operands of a product put
+sqrt(2) 2^-9 of its spread (1.4, normal inputs, He weights) on every element, 4e-3, and the largest of 3e4 elements is
+4.5 standard deviations out, 1.8e-2; the deltas carry two such roundings: 4e-2."""
+import pytest
+
+import harness as H
+from soklyn_b200 import configs
+from soklyn_b200.configs import NetSpec
+
+pytestmark = pytest.mark.gpu
+
+
+def _spec(name, dims, norm, act, prec, batch, optimiser="adam", dropout=0.0):
+    n = len(dims) - 2
+    return NetSpec(11, name, dims, (norm,) * n + ("disabled",), (act,) * n + ("identity",), (dropout,) * n + (0.0,), prec, "mse",
+                   "identity", optimiser, 1e-3, batch, "he_normal", "normal", "normal", dropout > 0)
+
+
+CASES = [
+    _spec("one_row_tile_cluster_of_8", (1024, 512, 256), "rms", "silu", "f16", 16),
+    _spec("k_steps_not_a_multiple_of_the_cluster", (456, 136, 72), "layer", "mish", "f16", 130, dropout=0.1),
+    _spec("two_row_tiles_one_row_in_the_last", (192, 264, 128), "disabled", "tanh", "bf16", 129, "sgd"),
+]
+
+
+@pytest.mark.parametrize("spec", CASES, ids=lambda s: s.name)
+def test_step_matches_oracle_at_the_edges(gpu_ctx, spec):
+    w = configs.make_weights(spec)
+    x, t, _ = configs.make_data(spec)
+    onet, _ = H.run_oracle(spec, w, x, t, 1)
+    dnet, _ = H.run_device(gpu_ctx, spec, w, x, t, 1)
+    H.compare_states(gpu_ctx, spec, dnet, onet, {"f32": 1e-5, "f16": 1e-2, "bf16": 4e-2}[spec.precision],
+                     skip=("mask", "dv_w", "dv_b", "dv_nw", "dv_nb"))
