@@ -415,6 +415,40 @@ bool layer_vec_ok(const sk_dense *L) {
     return L->N % 8 == 0;
 }
 
+// BatchNorm over the columns: column groups as wide as still give two blocks per SM (64 columns are a whole
+// 128-byte line of 16-bit rows, 16 a whole 32-byte sector), a cluster of up to 8 blocks per group.
+template <typename T, int V>
+cudaError_t launch_norm_cols(sk_ctx *c, const sk_dense *L, uint32_t batch, const ActDrop &ad) {
+    constexpr size_t kCacheBytes = 96 << 10;       // two blocks per SM
+    uint32_t split = 1, lanes = V == 8 ? 8 : 32;
+    while (split < 8 && batch >= split * 64) split *= 2;
+    auto blocks = [&] { return (size_t)((L->N + lanes * V - 1) / (lanes * V)) * split; };
+    while (V == 8 && lanes > 2 && blocks() < 2 * (size_t)c->num_sms) lanes /= 2;
+    const size_t bytes = ((size_t)batch + split - 1) / split * lanes * V * sizeof(T);
+    const bool cached = bytes <= kCacheBytes;
+    auto kernel = norm_cols_kernel<T, V>;
+    static uint64_t attr_set[4] = {0, 0, 0, 0};    // devices 0..255
+    const unsigned dev = (unsigned)c->device & 255u;
+    if (!(attr_set[dev >> 6] >> (dev & 63) & 1ull)) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCacheBytes);
+        if (e != cudaSuccess) return e;
+        attr_set[dev >> 6] |= 1ull << (dev & 63);
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks());
+    cfg.blockDim = dim3(kRowThreads);
+    cfg.dynamicSmemBytes = cached ? bytes : 0;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, (const T *)L->prenorm, (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered,
+                              (T *)L->preact, (T *)L->predrop, (T *)L->out, (T *)L->mask, (T *)L->norm_rstd, batch, L->N, lanes,
+                              ad, cached);
+}
+
 // ------------------------------------------------------------------------------------------
 template <typename T>
 int forward_impl(sk_ctx *c, const sk_dense *L, const void *x, uint32_t batch, uint32_t use_dropout, uint32_t step,
@@ -439,9 +473,9 @@ int forward_impl(sk_ctx *c, const sk_dense *L, const void *x, uint32_t batch, ui
     ProfScope ps(c, SK_PROF_NORM);
     ActDrop ad{L->act, use_dropout, seed, row_offset, L->leaky_coeff, L->mask_coeff};
     if (L->norm == SK_NORM_BATCH) {
-        norm_cols_kernel<T><<<(L->N + 31) / 32, kRowThreads, 0, c->stream>>>(
-            (const T *)L->prenorm, (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered, (T *)L->preact,
-            (T *)L->predrop, (T *)L->out, (T *)L->mask, (T *)L->norm_rstd, batch, L->N, ad);
+        const cudaError_t e = vec ? launch_norm_cols<T, 8>(c, L, batch, ad) : launch_norm_cols<T, 1>(c, L, batch, ad);
+        c->launches++;
+        return check_cuda(c, e, "forward norm");
     } else {
         const size_t cache_bytes = (size_t)L->N * sizeof(float);
         const bool cached = cache_bytes <= c->smem_optin;

@@ -5,6 +5,7 @@
 #pragma once
 
 #include "sk_epilogue.cuh"
+#include "sk_tc_ptx.cuh"
 
 namespace sk {
 
@@ -152,42 +153,99 @@ norm_rows_kernel(const T *__restrict__ prenorm, const T *__restrict__ norm_w, co
 }
 
 // BatchNorm (norm 3): statistics over the batch of each column, always from the batch
-// (ffn/forward.cu:74-126 with n = m). One block owns 32 adjacent columns so that every
-// access is a coalesced 32-wide row segment; 8 row lanes split the batch.
-template <typename T>
+// (ffn/forward.cu:74-126 with n = m). A cluster owns `lanes` x V adjacent columns and its blocks a contiguous
+// share of the rows each; a thread keeps V columns (128-bit accesses for V = 8), and the two sums (mean first,
+// then squared distances from it) are added over a block by shuffles and over the cluster through distributed
+// shared memory, in rank order. With `cached` the rows stay in shared memory between the three passes, so that
+// prenorm is read from memory once.
+template <typename T, int V>
 __global__ void __launch_bounds__(kRowThreads)
 norm_cols_kernel(const T *__restrict__ prenorm, const T *__restrict__ norm_w, const T *__restrict__ norm_b,
                  T *__restrict__ centered, T *__restrict__ preact, T *__restrict__ predrop, T *__restrict__ out,
-                 T *__restrict__ mask, T *__restrict__ rstd_out, uint32_t M, uint32_t N, ActDrop ad) {
-    __shared__ float red[8][33];
-    const uint32_t cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
-    const uint32_t col = blockIdx.x * 32 + cx;
-    const bool live = col < N;
-    auto reduce = [&](float v) {
-        red[ry][cx] = v;
-        __syncthreads();
-        float t = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) t += red[i][cx];
-        __syncthreads();
-        return t;
+                 T *__restrict__ mask, T *__restrict__ rstd_out, uint32_t M, uint32_t N, uint32_t lanes, ActDrop ad,
+                 bool cached) {
+    extern __shared__ __align__(16) uint8_t col_cache[];
+    __shared__ float red[kRowThreads / 32][32 * V];
+    __shared__ float total[2][32 * V];
+    T *cache = reinterpret_cast<T *>(col_cache);
+    const uint32_t rank = tc::cluster_rank(), split = tc::cluster_size();
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t cl = threadIdx.x % lanes, rl = threadIdx.x / lanes, row_lanes = kRowThreads / lanes, cols = lanes * V;
+    const uint32_t col = (blockIdx.x / split) * cols + cl * V;
+    const uint32_t r0 = (uint32_t)((uint64_t)rank * M / split), r1 = (uint32_t)((uint64_t)(rank + 1) * M / split);
+    const bool live = col < N;                     // V = 8 only with N % 8 == 0
+    auto fetch = [&](uint32_t r, bool from_cache, float (&x)[V]) {
+        load_run<T, V>(from_cache ? cache + (size_t)(r - r0) * cols + cl * V : prenorm + (size_t)r * N + col, true, x);
     };
-    float s = 0.0f;
-    if (live) for (uint32_t r = ry; r < M; r += 8) s += to_f32(prenorm[(size_t)r * N + col]);
-    const float mean = reduce(s) / (float)M;
-    float q = 0.0f;
-    if (live) for (uint32_t r = ry; r < M; r += 8) { const float d = to_f32(prenorm[(size_t)r * N + col]) - mean; q += d * d; }
-    const float rstd = rsqrtf(reduce(q) / (float)M + 1e-6f);
+    // sum over the rows of the whole batch, for every column of this thread
+    auto reduce = [&](float (&v)[V], uint32_t which) {
+#pragma unroll
+        for (int j = 0; j < V; ++j)
+            for (uint32_t o = 16; o >= lanes; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+        if (lane < lanes)
+#pragma unroll
+            for (int j = 0; j < V; ++j) red[warp][cl * V + j] = v[j];
+        __syncthreads();
+        for (uint32_t c = threadIdx.x; c < cols; c += kRowThreads) {
+            float t = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kRowThreads / 32; ++w) t += red[w][c];
+            total[which][c] = t;
+        }
+        tc::cluster_sync();
+#pragma unroll
+        for (int j = 0; j < V; ++j) v[j] = 0.0f;
+        for (uint32_t r = 0; r < split; ++r) {
+            const uint32_t at = tc::map_shared(tc::smem_u32(&total[which][cl * V]), r);
+#pragma unroll
+            for (int j = 0; j < V; ++j) v[j] += __uint_as_float(tc::ld_cluster_u32(at + 4 * j));
+        }
+    };
+    float mean[V], q[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) mean[j] = q[j] = 0.0f;
+    if (live)
+#pragma unroll 4
+        for (uint32_t r = r0 + rl; r < r1; r += row_lanes) {
+            float x[V];
+            fetch(r, false, x);
+#pragma unroll
+            for (int j = 0; j < V; ++j) mean[j] += x[j];
+            if (cached) store_run<T, V>(cache + (size_t)(r - r0) * cols + cl * V, true, x);   // a thread reads back its own rows only
+        }
+    reduce(mean, 0);
+#pragma unroll
+    for (int j = 0; j < V; ++j) mean[j] /= (float)M;
+    if (live)
+#pragma unroll 4
+        for (uint32_t r = r0 + rl; r < r1; r += row_lanes) {
+            float x[V];
+            fetch(r, cached, x);
+#pragma unroll
+            for (int j = 0; j < V; ++j) { const float d = x[j] - mean[j]; q[j] += d * d; }
+        }
+    reduce(q, 1);
+    tc::cluster_sync();                            // every total has been read: blocks may leave
     if (!live) return;
-    if (ry == 0) rstd_out[col] = from_f32<T>(rstd);
-    const float nw = to_f32(norm_w[col]), nb = to_f32(norm_b[col]);
-    for (uint32_t r = ry; r < M; r += 8) {
+    float scale[V], nb[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) q[j] = rsqrtf(q[j] / (float)M + 1e-6f);
+    if (rank == 0 && rl == 0) store_run<T, V>(rstd_out + col, true, q);
+    load_run<T, V>(norm_w + col, true, scale);
+    load_run<T, V>(norm_b + col, true, nb);
+#pragma unroll 1
+    for (uint32_t r = r0 + rl; r < r1; r += row_lanes) {
         const size_t idx = (size_t)r * N + col;
-        const float d = to_f32(prenorm[idx]) - mean;
-        centered[idx] = from_f32<T>(d);
-        float pre[1] = {round_to<T>(d * rstd * nw + nb)};
-        preact[idx] = from_f32<T>(pre[0]);
-        act_drop_store<T, 1>(ad, pre, r, col, idx, predrop, out, mask, false, 1);
+        float x[V], pre[V];
+        fetch(r, cached, x);
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            x[j] -= mean[j];
+            pre[j] = round_to<T>(x[j] * q[j] * scale[j] + nb[j]);
+        }
+        store_run<T, V>(centered + idx, true, x);
+        store_run<T, V>(preact + idx, true, pre);
+        act_drop_store<T, V>(ad, pre, r, col, idx, predrop, out, mask, true, V);
     }
 }
 
@@ -195,7 +253,7 @@ norm_cols_kernel(const T *__restrict__ prenorm, const T *__restrict__ norm_w, co
 // ranks (stats is f32 [2 x N]): phase 0 writes this shard's column sums of prenorm to stats[0];
 // phase 1 takes the summed stats[0] and writes this shard's sums of (x - mean)^2 to stats[1];
 // phase 2 takes both summed rows and does what norm_cols_kernel does after its reductions.
-// m_stat is the whole batch. Same thread layout as norm_cols_kernel.
+// m_stat is the whole batch. One block owns 32 adjacent columns, its 8 row lanes split the batch.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
 norm_cols_phase_kernel(uint32_t phase, float *__restrict__ stats, uint32_t m_stat, const T *__restrict__ prenorm,

@@ -23,6 +23,10 @@ CASES = [
     _spec("one_row_tile_cluster_of_8", (1024, 512, 256), "rms", "silu", "f16", 16),
     _spec("k_steps_not_a_multiple_of_the_cluster", (456, 136, 72), "layer", "mish", "f16", 130, dropout=0.1),
     _spec("two_row_tiles_one_row_in_the_last", (192, 264, 128), "disabled", "tanh", "bf16", 129, "sgd"),
+    _spec("batchnorm_five_rows", (64, 40, 16), "batch", "tanh", "f32", 5, "sgd"),
+    _spec("batchnorm_uneven_cluster", (128, 136, 10), "batch", "tanh", "f16", 1001),
+    _spec("batchnorm_scalar_columns", (77, 133, 10), "batch", "tanh", "f32", 65),
+    _spec("batchnorm_uncached_rows", (16, 64, 8), "batch", "sigmoid", "f32", 20011, "sgd"),
 ]
 
 
