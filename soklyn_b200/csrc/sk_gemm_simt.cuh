@@ -15,6 +15,7 @@
 #pragma once
 
 #include "sk_epilogue.cuh"
+#include "sk_tc_ptx.cuh"
 
 namespace sk {
 
@@ -34,7 +35,10 @@ __device__ __forceinline__ void load_guarded(const T *p, int valid, bool vec_ok,
 
 // BK: depth of one panel. These small tiles are used when the problem has few tiles (small or thin matrices),
 // where a block's time is one global-memory round trip per panel, not arithmetic: a deep panel (64 for the
-// 32 x 32 tile: eight elements per thread and operand in flight) divides the number of round trips.
+// 32 x 32 tile: eight elements per thread and operand in flight) divides the number of round trips. The 32 x 32
+// tile can also be worked on by a cluster (gridDim.z blocks): each takes a contiguous share of the panels, the
+// partial tiles are added through distributed shared memory in rank order, and every block finishes its share of
+// the rows. That changes the order of the sum, so it is for 16-bit operands only: f32 results keep the chain above.
 template <typename TA, typename TB, bool A_KCONTIG, bool B_NCONTIG, int BM, int BN, int TM, int TN, int BK, class Epi>
 __global__ void __launch_bounds__(kSimtThreads)
 gemm_simt_kernel(const TA *__restrict__ A, const TB *__restrict__ B, uint32_t M, uint32_t N, uint32_t K,
@@ -102,11 +106,15 @@ gemm_simt_kernel(const TA *__restrict__ A, const TB *__restrict__ B, uint32_t M,
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
 
-    fetch(0);
-    for (uint32_t k0 = 0; k0 < K; k0 += BK) {
+    constexpr bool kSplit = sizeof(TA) == 2 && BM * BN <= BK * (BM + PAD);   // the partial tile fits the A panel
+    const uint32_t split = kSplit ? gridDim.z : 1u, panels = (K + BK - 1) / BK;
+    const uint32_t first = (uint32_t)((uint64_t)blockIdx.z * panels / split) * BK;
+    const uint32_t end = min(K, (uint32_t)((uint64_t)(blockIdx.z + 1) * panels / split) * BK);
+    fetch(first);
+    for (uint32_t k0 = first; k0 < end; k0 += BK) {
         stage();
         __syncthreads();
-        if (k0 + BK < K) fetch(k0 + BK);
+        if (k0 + BK < end) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
             float a[TM], b[TN];
@@ -122,6 +130,34 @@ gemm_simt_kernel(const TA *__restrict__ A, const TB *__restrict__ B, uint32_t M,
         __syncthreads();
     }
 
+    if constexpr (kSplit) {
+        if (split > 1) {
+            float *part = &As[0][0];
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) part[(ty * TM + i) * BN + tx * TN + j] = acc[i][j];
+            tc::cluster_sync();
+            constexpr uint32_t kRuns = BM * BN / TN;
+            const uint32_t share = kRuns / split;
+            for (uint32_t u = t; u < share; u += kSimtThreads) {
+                const uint32_t at = (blockIdx.z * share + u) * TN, row = m0 + at / BN, col = n0 + at % BN;
+                if (row >= M || col >= N) continue;
+                float v[TN];
+#pragma unroll
+                for (int j = 0; j < TN; ++j) v[j] = 0.0f;
+                for (uint32_t r = 0; r < split; ++r) {
+                    const uint32_t p = tc::map_shared(tc::smem_u32(part + at), r);
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) v[j] += __uint_as_float(tc::ld_cluster_u32(p + 4 * j));
+                }
+                epi.template run<TN>(row, col, v, min((uint32_t)TN, N - col));
+            }
+            __syncwarp();
+            tc::cluster_sync();   // no block leaves while another still reads its partial tile
+            return;
+        }
+    }
     const uint32_t col0 = n0 + tx * TN;
     if (col0 >= N) return;
     const uint32_t ncols = min((uint32_t)TN, N - col0);
@@ -279,9 +315,22 @@ cudaError_t launch_gemm_simt(cudaStream_t stream, int num_sms, const TA *A, size
         gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 64, 64, 4, 4, 32, Epi>
             <<<grid, kSimtThreads, 0, stream>>>(A, B, M, N, K, lda, ldb, a_vec, b_vec, epi);
     } else {
-        dim3 grid((N + 31) / 32, (M + 31) / 32);
-        gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 32, 32, 2, 2, 64, Epi>
-            <<<grid, kSimtThreads, 0, stream>>>(A, B, M, N, K, lda, ldb, a_vec, b_vec, epi);
+        // a panel costs about a microsecond of round trip, a cluster's exchange about as much as two
+        const uint32_t panels = (K + 63) / 64;
+        uint32_t split = 1;
+        for (uint32_t s = 2; sizeof(TA) == 2 && s <= 8 && s <= panels && ctas(32, 32) * s <= 4 * (size_t)num_sms; s *= 2)
+            if ((panels + s - 1) / s + 2 < (split == 1 ? panels : (panels + split - 1) / split + 2)) split = s;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((N + 31) / 32, (M + 31) / 32, split);
+        cfg.blockDim = dim3(kSimtThreads);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = split;
+        cfg.attrs = attr;
+        cfg.numAttrs = split > 1 ? 1 : 0;
+        return cudaLaunchKernelEx(&cfg, gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 32, 32, 2, 2, 64, Epi>, A, B, M, N, K,
+                                  lda, ldb, a_vec, b_vec, epi);
     }
     return cudaGetLastError();
 }
