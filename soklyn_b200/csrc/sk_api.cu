@@ -277,20 +277,23 @@ cudaError_t launch_gemm_tc(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, co
                 : launch_tc_bn<T, A_MN, B_MN, 128, Epi>(c, ta, tb, M, N, K, epi, gate, group_n);
 }
 
-// ---- f32 operands on the tensor cores: three bf16 parts per operand, six partial products --------------
-// part[0] + part[1] + part[2] == x up to the last bit of f32 (each part holds the next 8 significant bits).
-__global__ void __launch_bounds__(256) split_bf16x3_kernel(const float *__restrict__ src, __nv_bfloat16 *__restrict__ p0,
-                                                            __nv_bfloat16 *__restrict__ p1, __nv_bfloat16 *__restrict__ p2,
-                                                            size_t len) {
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += stride) {
-        const float x = src[i];
-        const __nv_bfloat16 a = __float2bfloat16_rn(x);
-        const float r1 = x - __bfloat162float(a);
-        const __nv_bfloat16 b = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(b);
-        p0[i] = a; p1[i] = b; p2[i] = __float2bfloat16_rn(r2);
-    }
+// ---- operands in a layout TMA can fetch ------------------------------------------------------------------
+// Row pitch of a copy that TMA can fetch (whole 16-byte runs), and the bytes of one copy (256-byte aligned).
+inline size_t tma_pitch(size_t cols) { return (cols + 7) / 8 * 8; }
+inline size_t tma_copy_bytes(size_t rows, size_t cols) { return (rows * tma_pitch(cols) * 2 + 255) / 256 * 256; }
+
+template <typename S, int PARTS>
+cudaError_t launch_tma_copy(sk_ctx *c, const S *src, size_t rows, size_t cols, size_t ld, void *const *parts) {
+    const size_t groups = rows * (tma_pitch(cols) / 8);
+    size_t blocks = (groups + 255) / 256;
+    const size_t cap = (size_t)c->num_sms * 16;
+    if (blocks > cap) blocks = cap;
+    const bool vec = cols % 8 == 0 && ld * sizeof(S) % 16 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
+    TmaCopyParts dst{};
+    for (int i = 0; i < PARTS; ++i) dst.p[i] = parts[i];
+    tma_copy_kernel<S, PARTS><<<(unsigned)blocks, 256, 0, c->stream>>>(src, rows, (uint32_t)cols, ld, dst, vec);
+    c->launches++;
+    return cudaGetLastError();
 }
 
 // Smallest shape worth the split passes, and what the split copies need of the workspace.
@@ -301,19 +304,19 @@ cudaError_t launch_gemm_tc_split(sk_ctx *c, const float *A, size_t lda, const fl
                                  uint32_t K, const Epi &epi, bool *taken) {
     *taken = false;
     if (!c->f32_tensor || c->cc_major != 10 || !c->encode_tiled || !c->tc_err || !c->split_maps) return cudaSuccess;
-    if (!split_worthwhile(M, N, K) || lda % 8 || ldb % 8 || reinterpret_cast<uintptr_t>(A) % 16 || reinterpret_cast<uintptr_t>(B) % 16)
-        return cudaSuccess;
-    // elements of the row-major sources the GEMM touches
-    const size_t len_a = (size_t)(A_MN ? K : M) * lda, len_b = (size_t)(B_MN ? K : N) * ldb;
-    const size_t pad = 128;   // elements: keeps every part 256-byte aligned
-    const size_t ea = (len_a + pad - 1) / pad * pad, eb = (len_b + pad - 1) / pad * pad;
-    if ((3 * ea + 3 * eb) * sizeof(__nv_bfloat16) > c->workspace_bytes) return cudaSuccess;
-    __nv_bfloat16 *base = (__nv_bfloat16 *)c->workspace;
-    __nv_bfloat16 *pa[3] = {base, base + ea, base + 2 * ea}, *pb[3] = {base + 3 * ea, base + 3 * ea + eb, base + 3 * ea + 2 * eb};
-    auto blocks = [&](size_t len) { size_t b = (len + 1023) / 1024; const size_t cap = (size_t)c->num_sms * 16; return (unsigned)(b > cap ? cap : b); };
-    split_bf16x3_kernel<<<blocks(len_a), 256, 0, c->stream>>>(A, pa[0], pa[1], pa[2], len_a);
-    split_bf16x3_kernel<<<blocks(len_b), 256, 0, c->stream>>>(B, pb[0], pb[1], pb[2], len_b);
-    c->launches += 2;
+    if (!split_worthwhile(M, N, K)) return cudaSuccess;
+    // the row-major sources and their copies, whose row pitch is a whole number of 16-byte runs whatever the source's
+    const size_t rows_a = A_MN ? K : M, cols_a = A_MN ? M : K, rows_b = B_MN ? K : N, cols_b = B_MN ? N : K;
+    const size_t bytes_a = tma_copy_bytes(rows_a, cols_a), bytes_b = tma_copy_bytes(rows_b, cols_b);
+    if (3 * (bytes_a + bytes_b) > c->workspace_bytes) return cudaSuccess;
+    uint8_t *base = (uint8_t *)c->workspace;
+    void *pa[3] = {base, base + bytes_a, base + 2 * bytes_a};
+    void *pb[3] = {base + 3 * bytes_a, base + 3 * bytes_a + bytes_b, base + 3 * bytes_a + 2 * bytes_b};
+    cudaError_t e;
+    if ((e = launch_tma_copy<float, 3>(c, A, rows_a, cols_a, lda, pa)) != cudaSuccess) return e;
+    if ((e = launch_tma_copy<float, 3>(c, B, rows_b, cols_b, ldb, pb)) != cudaSuccess) return e;
+    lda = tma_pitch(cols_a);
+    ldb = tma_pitch(cols_b);
     const uint32_t sms = tc_sms(c);
     constexpr uint32_t bn = 128;   // the split kernel's tile: four accumulator buffers of 128 columns
     TcSplitMaps maps;
@@ -323,8 +326,7 @@ cudaError_t launch_gemm_tc_split(sk_ctx *c, const float *A, size_t lda, const fl
         if (!ok_a || !ok_b) return cudaErrorInvalidValue;
     }
     TcSplitMaps *dev = c->split_maps + (c->split_slot++ % kSplitMapSlots);
-    cudaError_t e = cudaMemcpyAsync(dev, &maps, sizeof maps, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(dev, &maps, sizeof maps, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess) return e;
     *taken = true;
     const uint32_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + bn - 1) / bn);
     const uint32_t grid = tiles < sms ? tiles : sms;
@@ -341,6 +343,40 @@ cudaError_t launch_gemm_tc_split(sk_ctx *c, const float *A, size_t lda, const fl
     return cudaGetLastError();
 }
 
+// 16-bit operands whose base or row pitch TMA cannot fetch (widths that are no multiple of 8, 10-wide heads): they
+// are copied to a fetchable pitch in the workspace first. Worth it once the FFMA kernel would take longer than the
+// copies and the fixed cost of the tensor-core kernel: measured, its small tiles run at about 8 TFLOP/s of the
+// padded tile (300 x 1001 x 777: 56 us, 8192 x 10 x 512: 25 us), a copy costs 2 us and its traffic, the
+// tensor-core kernel about 10 us.
+template <typename T, bool A_MN, bool B_MN, class Epi>
+cudaError_t launch_gemm_tc_copied(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, const T *B, size_t ldb, uint32_t M, uint32_t N,
+                                  uint32_t K, const Epi &epi, bool *taken) {
+    *taken = false;
+    if (c->gemm_engine == 1 || c->cc_major != 10 || !c->encode_tiled || !c->tc_err) return cudaSuccess;
+    auto fetchable = [](const T *p, size_t ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 8 == 0; };
+    const bool copy_a = !fetchable(A, lda), copy_b = !fetchable(B, ldb);
+    const size_t rows_a = A_MN ? K : M, cols_a = A_MN ? M : K, rows_b = B_MN ? K : N, cols_b = B_MN ? N : K;
+    const size_t bytes_a = copy_a ? tma_copy_bytes(rows_a, cols_a) : 0, bytes_b = copy_b ? tma_copy_bytes(rows_b, cols_b) : 0;
+    if (bytes_a + bytes_b > c->workspace_bytes) return cudaSuccess;
+    auto padded = [](double v) { return (double)(((uint64_t)v + 31) / 32 * 32); };
+    const double ffma_us = 6.0 + 2e-6 * padded(M) * padded(N) * K / 8.0;
+    const double copies_us = 10.0 + 2.0 * (copy_a + copy_b) + 2.0 * (double)(bytes_a + bytes_b) / 3e6;
+    if (ffma_us <= copies_us) return cudaSuccess;
+    cudaError_t e;
+    if (copy_a) {
+        void *to[1] = {c->workspace};
+        if ((e = launch_tma_copy<T, 1>(c, A, rows_a, cols_a, lda, to)) != cudaSuccess) return e;
+        A = (const T *)to[0]; lda = tma_pitch(cols_a);
+    }
+    if (copy_b) {
+        void *to[1] = {(uint8_t *)c->workspace + bytes_a};
+        if ((e = launch_tma_copy<T, 1>(c, B, rows_b, cols_b, ldb, to)) != cudaSuccess) return e;
+        B = (const T *)to[0]; ldb = tma_pitch(cols_b);
+    }
+    *taken = true;
+    return launch_gemm_tc<T, A_MN, B_MN, Epi>(c, dtype, A, lda, B, ldb, M, N, K, epi);
+}
+
 // Engine choice for one product of the DenseBlock path.
 template <typename TA, typename TB, bool A_KCONTIG, bool B_NCONTIG, class Epi>
 cudaError_t run_gemm(sk_ctx *c, uint32_t dtype, const TA *A, size_t lda, const TB *B, size_t ldb, uint32_t M, uint32_t N,
@@ -350,6 +386,11 @@ cudaError_t run_gemm(sk_ctx *c, uint32_t dtype, const TA *A, size_t lda, const T
             return launch_gemm_tc<TA, !A_KCONTIG, B_NCONTIG, Epi>(c, dtype, A, lda, B, ldb, M, N, K, epi, gate);
     }
     if (gate.flags) return cudaErrorNotSupported;   // only the tensor-core kernel can wait for rows in flight
+    if constexpr (std::is_same<TA, TB>::value && !std::is_same<TA, float>::value) {
+        bool taken = false;
+        const cudaError_t e = launch_gemm_tc_copied<TA, !A_KCONTIG, B_NCONTIG, Epi>(c, dtype, A, lda, B, ldb, M, N, K, epi, &taken);
+        if (taken || e != cudaSuccess) return e;
+    }
     if constexpr (std::is_same<TA, float>::value && std::is_same<TB, float>::value) {
         bool taken = false;
         const cudaError_t e = launch_gemm_tc_split<!A_KCONTIG, B_NCONTIG, Epi>(c, A, lda, B, ldb, M, N, K, epi, &taken);
@@ -579,12 +620,13 @@ int hidden_error_impl(sk_ctx *c, const sk_dense *cur, const sk_dense *next, uint
     ProfScope ps(c, SK_PROF_GEMM_DX);
     cudaError_t e;
     // kernels specialised for the activation / normalisation pairs of the wide and the classifier networks
-    if (!f32 && cur->act == SK_ACT_SILU && cur->norm == SK_NORM_RMS) {
+    // (they take 128-bit rows only)
+    if (!f32 && epi.vec_ok && cur->act == SK_ACT_SILU && cur->norm == SK_NORM_RMS) {
         EpiHidden<T, SK_ACT_SILU, SK_NORM_RMS> se;
         static_assert(sizeof(se) == sizeof(epi), "specialised functor has the same fields");
         memcpy(&se, &epi, sizeof se);
         e = run_gemm<T, T, true, false>(c, cur->dtype, dy, ec, wn, ec, batch, cur->N, ec, se, gate);
-    } else if (!f32 && cur->act == SK_ACT_MISH && cur->norm == SK_NORM_LAYER) {
+    } else if (!f32 && epi.vec_ok && cur->act == SK_ACT_MISH && cur->norm == SK_NORM_LAYER) {
         EpiHidden<T, SK_ACT_MISH, SK_NORM_LAYER> se;
         memcpy(&se, &epi, sizeof se);
         e = run_gemm<T, T, true, false>(c, cur->dtype, dy, ec, wn, ec, batch, cur->N, ec, se, gate);
@@ -696,7 +738,7 @@ int backward_update_impl(sk_ctx *c, const sk_dense *L, const void *x, uint32_t b
     if (f32) {
         rc = check_cuda(c, run_gemm<T, float, false, true>(c, L->dtype, (const T *)x, L->K, L->d_prenorm,
                                                                     L->N, L->K, L->N, batch, epi), "weight gradient gemm");
-    } else if (lin.kind == SK_OPT_ADAM && L->regu == SK_REGU_NONE) {   // specialised: Adam, no regularisation
+    } else if (epi.vec_ok && lin.kind == SK_OPT_ADAM && L->regu == SK_REGU_NONE) {   // specialised: Adam, no regularisation, 128-bit rows
         EpiWeightUpdate<T, SK_OPT_ADAM, SK_REGU_NONE> se;
         static_assert(sizeof(se) == sizeof(epi), "specialised functor has the same fields");
         memcpy(&se, &epi, sizeof se);
@@ -1004,7 +1046,7 @@ int sk_ctx_create(int device, uint32_t tile_dim, void *stream, int create_stream
         else c->dp_counters = nullptr;
         if (cudaMalloc(&c->split_maps, kSplitMapSlots * sizeof(TcSplitMaps)) != cudaSuccess) c->split_maps = nullptr;
     }
-    if (workspace_bytes == 0) workspace_bytes = (size_t)64 << 20;
+    if (workspace_bytes == 0) workspace_bytes = (size_t)256 << 20;
     if (cudaMalloc(&c->workspace, workspace_bytes) != cudaSuccess) {
         if (c->own_stream) cudaStreamDestroy(c->stream);
         if (c->tc_err) cudaFree(c->tc_err);

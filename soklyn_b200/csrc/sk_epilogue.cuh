@@ -11,6 +11,9 @@
 //       (bias, normalisation weights) once, prefetch() issues the raw loads of the next row's
 //       run before the current one is finished, finish() consumes them. These are used only
 //       when every tensor allows 128-bit accesses (vec_ok) and the run has all 8 columns.
+//   prefetch1(row, col, p) / finish1(row, col, acc, p) one element at a time, for tensors without
+//       128-bit rows: a warp takes 32 adjacent columns, so that its scalar accesses are coalesced,
+//       and several rows at once, so that their loads are in flight together.
 #pragma once
 
 #include "sk_device.cuh"
@@ -148,6 +151,9 @@ template <typename T> struct EpiForward {
     __device__ __forceinline__ void finish(uint32_t row, uint32_t col0, const float (&acc)[8], const Pre &, const Cols &c) const {
         core<8>(row, col0, acc, c.b);
     }
+    using Pre1 = NoPre;
+    __device__ __forceinline__ void prefetch1(uint32_t, uint32_t, Pre1 &) const {}
+    __device__ __forceinline__ void finish1(uint32_t row, uint32_t col, float acc, const Pre1 &) const { one(row, col, acc); }
 };
 
 // ---- hidden delta: S = dY_next . W_next^T, times act', times mask, normalisation backward ----
@@ -180,19 +186,33 @@ template <typename T, int ACT = -1, int NORM = -1> struct EpiHidden {
     __device__ __forceinline__ uint32_t A() const { return ACT >= 0 ? (uint32_t)ACT : act; }
     __device__ __forceinline__ uint32_t Nm() const { return NORM >= 0 ? (uint32_t)NORM : norm; }
 
-    __device__ __forceinline__ void one(uint32_t row, uint32_t col, float s) const {
+    struct Pre1 { T pd, pa, mk, xv, r; };
+    __device__ __forceinline__ void prefetch1(uint32_t row, uint32_t col, Pre1 &p) const {
         const size_t idx = (size_t)row * N + col;
-        const float delta = to_f32(mask[idx]) *
-                            activation_derivative(act, s * acc_scale, to_f32(predrop[idx]), to_f32(preact[idx]), leaky);
+        p.pd = predrop[idx];
+        p.pa = preact[idx];
+        p.mk = mask[idx];
+        if (Nm() == 1) p.xv = prenorm[idx];
+        else if (Nm() >= 2) p.xv = centered[idx];
+        if (Nm()) p.r = rstd[Nm() == 3 ? col : row];
+    }
+    __device__ __forceinline__ void finish1(uint32_t row, uint32_t col, float s, const Pre1 &p) const {
+        const size_t idx = (size_t)row * N + col;
+        const float delta = to_f32(p.mk) * activation_derivative(A(), s * acc_scale, to_f32(p.pd), to_f32(p.pa), leaky);
         grad[idx] = delta;
-        const float r = norm ? to_f32(rstd[norm == 3 ? col : row]) : 0.0f;
-        const float pv = norm == 1 ? to_f32(prenorm[idx]) : 0.0f;
-        const float cv = norm >= 2 ? to_f32(centered[idx]) : 0.0f;
-        const NormGrad g = norm_gradients(norm, delta, pv, cv, r, norm_w[col], inv_n, inv_m);
+        const float r = Nm() ? to_f32(p.r) : 0.0f;
+        const float pv = Nm() == 1 ? to_f32(p.xv) : 0.0f;
+        const float cv = Nm() >= 2 ? to_f32(p.xv) : 0.0f;
+        const NormGrad g = norm_gradients(Nm(), delta, pv, cv, r, norm_w[col], inv_n, inv_m);
         d_prenorm[idx] = g.d_prenorm;
         d_norm_w[idx] = g.d_norm_w;
         d_norm_b[idx] = g.d_norm_b;
         if (d_prenorm_lp) d_prenorm_lp[idx] = from_f32<T>(g.d_prenorm * kLpScale);
+    }
+    __device__ __forceinline__ void one(uint32_t row, uint32_t col, float s) const {
+        Pre1 p;
+        prefetch1(row, col, p);
+        finish1(row, col, s, p);
     }
 
     // vector path on unpacked inputs of one run. nw: normalisation weights of the columns,
@@ -274,6 +294,7 @@ template <typename T, int ACT = -1, int NORM = -1> struct EpiHidden {
 
     // the specialised kernels are small enough to be unrolled with two passes of loads in flight
     static constexpr bool kPingPong = ACT >= 0 && NORM >= 0;
+    static constexpr bool kVecOnly = kPingPong;
     static constexpr int kGroup = kPingPong ? 2 : 1;
     struct Cols { float nw[8], rs[8]; };
     struct Pre { Pack<T, 8> pd, pa, mk, xv; T rrow; };
@@ -406,6 +427,7 @@ template <typename T, int KIND = -1, int REGU = -1> struct EpiWeightUpdate {
     }
 
     static constexpr bool kPingPong = KIND >= 0 && REGU >= 0;
+    static constexpr bool kVecOnly = kPingPong;
     struct Cols {};
     struct Pre { Pack<float, 8> p, v, m; };
     __device__ __forceinline__ void cols(uint32_t, Cols &) const {}
@@ -427,6 +449,18 @@ template <typename T, int KIND = -1, int REGU = -1> struct EpiWeightUpdate {
         store_run<float, 8>(dm + idx, true, m);
         store_run<float, 8>(master + idx, true, p);
         if ((void *)w != (void *)master) store_run<T, 8>(w + idx, true, p);
+    }
+    struct Pre1 { float p, v, m; };
+    __device__ __forceinline__ void prefetch1(uint32_t row, uint32_t col, Pre1 &q) const {
+        const size_t idx = (size_t)row * N + col;
+        q.p = master[idx]; q.v = dv[idx]; q.m = dm[idx];
+    }
+    __device__ __forceinline__ void finish1(uint32_t row, uint32_t col, float acc, const Pre1 &q) const {
+        const size_t idx = (size_t)row * N + col;
+        float v = q.v, m = q.m;
+        const float p = optimiser_step(q.p, v, m, acc * gscale, opt, hyp, true);
+        dv[idx] = v; dm[idx] = m; master[idx] = p;
+        if ((void *)w != (void *)master) w[idx] = from_f32<T>(p);
     }
 };
 
@@ -453,6 +487,12 @@ struct EpiStoreF32 {
     __device__ __forceinline__ void finish(uint32_t row, uint32_t col0, const float (&acc)[8], const Pre &, const Cols &) const {
         run<8>(row, col0, acc, 8);
     }
+    using Pre1 = NoPre;
+    __device__ __forceinline__ void prefetch1(uint32_t, uint32_t, Pre1 &) const {}
+    __device__ __forceinline__ void finish1(uint32_t row, uint32_t col, float acc, const Pre1 &) const {
+        const float v[1] = {acc};
+        run<1>(row, col, v, 1);
+    }
 };
 
 // ---- scaled store in the storage type (16-bit gradient payload of the data-parallel exchange) ----
@@ -477,6 +517,12 @@ template <typename T> struct EpiStoreScaled {
     __device__ __forceinline__ void prefetch(uint32_t, uint32_t, Pre &) const {}
     __device__ __forceinline__ void finish(uint32_t row, uint32_t col0, const float (&acc)[8], const Pre &, const Cols &) const {
         run<8>(row, col0, acc, 8);
+    }
+    using Pre1 = NoPre;
+    __device__ __forceinline__ void prefetch1(uint32_t, uint32_t, Pre1 &) const {}
+    __device__ __forceinline__ void finish1(uint32_t row, uint32_t col, float acc, const Pre1 &) const {
+        const float v[1] = {acc};
+        run<1>(row, col, v, 1);
     }
 };
 

@@ -38,6 +38,7 @@ constexpr int kTcBK = 64;           // K depth of one stage: 64 x 2 B = one 128-
 constexpr int kTcEpiWarps = 8;
 constexpr int kTcThreads = (2 + kTcEpiWarps) * 32;
 constexpr int kTcABytes = kTcBM * kTcBK * 2;
+constexpr uint32_t kRows1 = 4;      // rows whose loads are in flight together in an element-wise epilogue
 
 template <int BN> struct TcShape {
     static constexpr int kBBytes = BN * kTcBK * 2;
@@ -59,6 +60,9 @@ template <class Epi> struct EpiAcc<Epi, std::enable_if_t<Epi::kHasAcc>> { static
 // Functors whose body is small enough to exist four times declare kPingPong = true.
 template <class Epi, class = void> struct EpiPingPong { static constexpr bool value = false; };
 template <class Epi> struct EpiPingPong<Epi, decltype((void)Epi::kPingPong)> { static constexpr bool value = Epi::kPingPong; };
+// Functors that are used with vec_ok only (the specialised ones) declare kVecOnly: no element-wise epilogue is built.
+template <class Epi, class = void> struct VecOnly { static constexpr bool value = false; };
+template <class Epi> struct VecOnly<Epi, decltype((void)Epi::kVecOnly)> { static constexpr bool value = Epi::kVecOnly; };
 
 enum : int { kTcErrProducer = 1, kTcErrMma = 2, kTcErrEpilogue = 3, kTcErrGate = 4 };
 
@@ -358,8 +362,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (n0 + c0 >= N) break;              // uniform per warp
                 const uint32_t col = n0 + c0 + cc;
                 const bool col_ok = col < N;
-                const uint32_t ncols = col_ok ? min(8u, N - col) : 0u;
-                const bool fast = epi.vec_ok && ncols == 8;   // else: ragged right edge, unaligned tensors
+                const bool fast = epi.vec_ok && col_ok;       // vec_ok: N is a multiple of 8, a run has all columns or none
                 if (fast && !have) {
                     epi.cols(col, cols);
 #pragma unroll
@@ -377,6 +380,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                 for (int j = 0; j < 32; ++j) buf[lane * 33 + j] = v[j];
                 __syncwarp();
+                if (!VecOnly<Epi>::value && !epi.vec_ok) {   // one element per lane, kRows1 rows of loads in flight
+                    const uint32_t col1 = n0 + c0 + lane, rows = min(32u, M - min(M, m0 + quarter * 32));
+#pragma unroll 1
+                    for (uint32_t r0 = 0; r0 < rows && col1 < N; r0 += kRows1) {
+                        typename Epi::Pre1 p1[kRows1];
+#pragma unroll
+                        for (uint32_t r = 0; r < kRows1; ++r)
+                            if (r0 + r < rows) epi.prefetch1(m0 + quarter * 32 + r0 + r, col1, p1[r]);
+#pragma unroll
+                        for (uint32_t r = 0; r < kRows1; ++r)
+                            if (r0 + r < rows) epi.finish1(m0 + quarter * 32 + r0 + r, col1, buf[(r0 + r) * 33 + lane], p1[r]);
+                    }
+                    __syncwarp();
+                    continue;
+                }
                 bool have_n = false;
                 typename EpiAcc<Epi>::type sums;
                 if constexpr (EpiAcc<Epi>::value) epi.acc_init(sums);
@@ -403,12 +421,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                         for (int j = 0; j < 8; ++j) r[j] = buf[rr * 33 + cc + j];
                         if (col_ok && row < M) {
-                            if (fast) {
-                                if constexpr (EpiAcc<Epi>::value) epi.finish(row, col, r, cur[g], cols, sums);
-                                else epi.finish(row, col, r, cur[g], cols);
-                            } else {
-                                epi.template run<8>(row, col, r, ncols);
-                            }
+                            if constexpr (EpiAcc<Epi>::value) epi.finish(row, col, r, cur[g], cols, sums);
+                            else epi.finish(row, col, r, cur[g], cols);
                         }
                     }
                 };
@@ -571,22 +585,46 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     // a block whose waits ran out has filled in no valid tile: the cluster then writes nothing
     bool valid = true;
     for (uint32_t r = 0; r < split; ++r) valid = valid && tc::ld_cluster_u32(tc::map_shared(tc::smem_u32(gave_up), r)) == 0;
-    if (warp >= 2 && valid) {
+    if (!VecOnly<Epi>::value && warp >= 2 && valid && !epi.vec_ok) {   // one element per lane
+        const uint32_t rows = min((uint32_t)kTcBM, M - m0), step = kTcEpiWarps * split;
+#pragma unroll 1
+        for (uint32_t c = lane; c < BN && n0 + c < N; c += 32) {
+            const uint32_t base = tc::smem_u32(partial) + ((c & 4) / 4 * (BN / 2) + c / 8 * 4 + (c & 3)) * 4;
+#pragma unroll 1
+            for (uint32_t r0 = (warp - 2) * split + rank; r0 < rows; r0 += step * kRows1) {
+                typename Epi::Pre1 p1[kRows1];
+                float v[kRows1];
+#pragma unroll
+                for (uint32_t r = 0; r < kRows1; ++r) {
+                    v[r] = 0.0f;
+                    if (r0 + r * step < rows) epi.prefetch1(m0 + r0 + r * step, n0 + c, p1[r]);
+                }
+                for (uint32_t s = 0; s < split; ++s) {
+                    const uint32_t from = tc::map_shared(base, s);
+#pragma unroll
+                    for (uint32_t r = 0; r < kRows1; ++r)
+                        if (r0 + r * step < rows) v[r] += __uint_as_float(tc::ld_cluster_u32(from + (r0 + r * step) * kPitch * 4));
+                }
+#pragma unroll
+                for (uint32_t r = 0; r < kRows1; ++r)
+                    if (r0 + r * step < rows) epi.finish1(m0 + r0 + r * step, n0 + c, v[r], p1[r]);
+            }
+        }
+    } else if (warp >= 2 && valid) {
         constexpr uint32_t kLanesRow = BN / 8, kRows = 32 / kLanesRow;      // rows per warp and pass: 1 (BN = 256) or 2
         const uint32_t units = (min((uint32_t)kTcBM, M - m0) + kRows - 1) / kRows, run = lane % kLanesRow;
-        const uint32_t col = n0 + run * 8, ncols = col < N ? min(8u, N - col) : 0u;
-        const bool fast = epi.vec_ok && ncols == 8;
+        const uint32_t col = n0 + run * 8;
         const uint32_t base = tc::smem_u32(partial) + run * 16;
         typename Epi::Cols cols;
-        if (fast) epi.cols(col, cols);
+        if (col < N) epi.cols(col, cols);
         typename EpiAcc<Epi>::type sums;
         if constexpr (EpiAcc<Epi>::value) epi.acc_init(sums);
 #pragma unroll 1
         for (uint32_t u = (warp - 2) * split + rank; u < units; u += kTcEpiWarps * split) {
             const uint32_t row = m0 + u * kRows + lane / kLanesRow;
-            if (row >= M || ncols == 0) continue;
+            if (row >= M || col >= N) continue;
             typename Epi::Pre pre;
-            if (fast) epi.prefetch(row, col, pre);
+            epi.prefetch(row, col, pre);
             const uint32_t at = base + (row - m0) * kPitch * 4;
             float v[8];
 #pragma unroll
@@ -600,12 +638,8 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                 v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
                 v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
             }
-            if (fast) {
-                if constexpr (EpiAcc<Epi>::value) epi.finish(row, col, v, pre, cols, sums);
-                else epi.finish(row, col, v, pre, cols);
-            } else {
-                epi.template run<8>(row, col, v, ncols);
-            }
+            if constexpr (EpiAcc<Epi>::value) epi.finish(row, col, v, pre, cols, sums);
+            else epi.finish(row, col, v, pre, cols);
         }
         // running sums: one slab per warp of the cluster, over all its rows of the tile
         if constexpr (EpiAcc<Epi>::value) {

@@ -23,6 +23,9 @@ CASES = [
     _spec("one_row_tile_cluster_of_8", (1024, 512, 256), "rms", "silu", "f16", 16),
     _spec("k_steps_not_a_multiple_of_the_cluster", (456, 136, 72), "layer", "mish", "f16", 130, dropout=0.1),
     _spec("two_row_tiles_one_row_in_the_last", (192, 264, 128), "disabled", "tanh", "bf16", 129, "sgd"),
+    _spec("odd_widths_copied", (333, 417, 203, 10), "layer", "mish", "f16", 301),
+    _spec("odd_widths_copied_rms", (515, 266, 1001, 7), "rms", "silu", "f16", 257, dropout=0.3),
+    _spec("odd_widths_persistent_tiles", (77, 2557, 130), "disabled", "sigmoid", "f16", 1950, "sgd"),
     _spec("batchnorm_five_rows", (64, 40, 16), "batch", "tanh", "f32", 5, "sgd"),
     _spec("batchnorm_uneven_cluster", (128, 136, 10), "batch", "tanh", "f16", 1001),
     _spec("batchnorm_scalar_columns", (77, 133, 10), "batch", "tanh", "f32", 65),
@@ -39,3 +42,16 @@ def test_step_matches_oracle_at_the_edges(gpu_ctx, spec):
     dnet, _ = H.run_device(gpu_ctx, spec, w, x, t, 1)
     H.compare_states(gpu_ctx, spec, dnet, onet, {"f32": 1e-5, "f16": 1e-2, "bf16": 4e-2}[spec.precision],
                      skip=("mask", "dv_w", "dv_b", "dv_nw", "dv_nb"))
+
+
+def test_f32_tensor_core_option_takes_odd_widths(gpu_ctx):
+    spec = _spec("f32_tensor_cores_odd", (515, 1030, 333), "rms", "silu", "f32", 601, "sgd")
+    w = configs.make_weights(spec)
+    x, t, _ = configs.make_data(spec)
+    onet, _ = H.run_oracle(spec, w, x, t, 1)
+    try:
+        gpu_ctx.set_f32_tensor_cores(True)
+        dnet, _ = H.run_device(gpu_ctx, spec, w, x, t, 1)
+    finally:
+        gpu_ctx.set_f32_tensor_cores(False)
+    H.compare_states(gpu_ctx, spec, dnet, onet, 5e-5, skip=("mask", "dv_w", "dv_b", "dv_nw", "dv_nb"))
