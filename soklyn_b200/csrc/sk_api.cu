@@ -401,6 +401,9 @@ cudaError_t run_gemm(sk_ctx *c, uint32_t dtype, const TA *A, size_t lda, const T
 
 inline bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 constexpr uint32_t kSmallBatchRows = 256;   // up to here column sums and the vector step share one launch
+// Elements up to which a cluster per column group takes them in one launch: measured 9 against 13 us at 512 x 1024, but
+// 23 against 20 us at 4096 x 1024 and 84 against 55 us at 65536 x 1024, where the plain grid streams better.
+constexpr uint64_t kColsumClusterMax = 1u << 21;
 constexpr uint32_t kHandoverMinRows = 512;   // below this a separate column-sum pass costs as little as the heavier dX epilogue (measured: 0.4 % of a step gained at 512 rows, 1.4 % at 1024, none at 256)
 constexpr uint32_t kColsumFold = 8;   // slabs the per-32-row column sums of the dX epilogue are folded into
 
@@ -523,7 +526,12 @@ int forward_impl(sk_ctx *c, const sk_dense *L, const void *x, uint32_t batch, ui
         // rows stream straight from global memory (the second pass hits L2): no shared memory,
         // so eight blocks fit an SM; the shared-memory row cache is kept for rows of odd length
         const bool use_cache = cached && !vec;
-        norm_rows_kernel<T><<<batch, kRowThreads, use_cache ? cache_bytes : 0, c->stream>>>(
+        // few long rows (16 x 16384: 14 us with 256 threads, 7 with 1024): four times the threads on each; rows of at
+        // most 1024 elements have work for 128 threads, and twice as many of them fit an SM
+        const bool few = batch < (uint32_t)c->num_sms && L->N >= 4096, brief = L->N <= 1024;
+        const uint32_t threads = few ? 1024 : brief ? 128 : kRowThreads;
+        auto kernel = few ? norm_rows_kernel<T, 1024> : brief ? norm_rows_kernel<T, 128> : norm_rows_kernel<T, kRowThreads>;
+        kernel<<<batch, threads, use_cache ? cache_bytes : 0, c->stream>>>(
             (const T *)L->prenorm, (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered, (T *)L->preact,
             (T *)L->predrop, (T *)L->out, (T *)L->mask, (T *)L->norm_rstd, L->N, L->norm, ad, vec, use_cache);
     }
@@ -701,7 +709,7 @@ int vector_update_launch(sk_ctx *c, const sk_dense *L, const float *partial, uin
 }
 
 // Column sums + bias / normalisation-parameter step of a block. Small batches take both in one
-// launch; otherwise the sums come from the dX epilogue or the two-stage column-sum kernel.
+// launch, so do middle-sized tensors and the partial sums of the dX epilogue; large ones go through two stages.
 template <typename T>
 int column_sums_and_vector_update(sk_ctx *c, const sk_dense *L, uint32_t batch, const Optim &lin, const Optim &nrm,
                                   const Hyper &hyp) {
@@ -713,6 +721,34 @@ int column_sums_and_vector_update(sk_ctx *c, const sk_dense *L, uint32_t batch, 
                                                                              L->N, vector_params<T>(L, lin, nrm, hyp));
         c->launches++;
         return check_cuda(c, cudaGetLastError(), "column sums + bias / norm parameter step");
+    }
+    if (handed || (uint64_t)batch * L->N <= kColsumClusterMax) {
+        c->fused_colsum_key = nullptr;
+        // handed over: one slab [3 x N] per group of rows in the workspace
+        const float *ws = (const float *)c->workspace, *p = handed ? ws : L->d_prenorm, *w = handed ? ws + L->N : L->d_norm_w,
+                    *b = handed ? ws + 2 * (size_t)L->N : L->d_norm_b;
+        const uint32_t rows = handed ? c->fused_colsum_groups : batch;
+        const size_t ld = handed ? 3 * (size_t)L->N : L->N;
+        ProfScope ps(c, SK_PROF_COLSUM);
+        const VectorParams<T> P = vector_params<T>(L, lin, nrm, hyp);
+        const bool vec = L->N % 4 == 0 && aligned16(p) && aligned16(w) && aligned16(b);
+        uint32_t split = 1, lanes = vec ? 8 : 32;
+        while (split < 8 && rows >= split * 256) split *= 2;
+        auto blocks = [&] { return (size_t)((L->N + lanes * (vec ? 4 : 1) - 1) / (lanes * (vec ? 4 : 1))) * split; };
+        // narrower column groups while the chip is not full: down to whole 32-byte sectors, or the columns there are
+        while (vec ? lanes > 2 && blocks() < (size_t)c->num_sms : lanes > 8 && lanes / 2 >= L->N) lanes /= 2;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)blocks());
+        cfg.blockDim = dim3(kColThreads);
+        cfg.stream = c->stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        c->launches++;
+        return check_cuda(c, cudaLaunchKernelEx(&cfg, vec ? colsum_cluster_kernel<T, 4> : colsum_cluster_kernel<T, 1>, p, w, b, rows,
+                                                L->N, ld, lanes, P), "column sums + bias / norm parameter step");
     }
     int rc = SK_OK;
     uint32_t nslabs = 0;
@@ -1025,9 +1061,15 @@ int sk_ctx_create(int device, uint32_t tile_dim, void *stream, int create_stream
         c->own_stream = true;
     }
     const int optin = (int)c->smem_optin;
-    cudaFuncSetAttribute(sk::norm_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-    cudaFuncSetAttribute(sk::norm_rows_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-    cudaFuncSetAttribute(sk::norm_rows_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<float, kRowThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<float, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<__half, kRowThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<__half, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<__half, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<__nv_bfloat16, kRowThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<__nv_bfloat16, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(sk::norm_rows_kernel<__nv_bfloat16, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     c->cc_major = prop.major;
     if (c->cc_major == 10) query_cluster_blocks(c);
     if (const char *env = getenv("SK_TC_GROUP_N")) { const int v = atoi(env); if (v >= 1 && v <= 64) c->tc_group_n = (uint32_t)v; }

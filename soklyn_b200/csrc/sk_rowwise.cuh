@@ -10,6 +10,7 @@
 namespace sk {
 
 constexpr int kRowThreads = 256;
+constexpr int kColThreads = 512;   // column sums on clusters: there are fewer column groups than warp slots
 
 struct ActDrop {
     uint32_t act, use_dropout, seed, row_offset;
@@ -49,8 +50,8 @@ __device__ __forceinline__ void act_drop_store(const ActDrop &ad, const float (&
 // when `cached`), writes centered, preact, predrop, out, (mask) and rstd[row]. The output loop
 // is kept rolled so that the activation code exists once (instruction-cache footprint).
 // Reference: ffn/forward.cu:44-73 (RMS, products in T arithmetic), :74-126 (LayerNorm).
-template <typename T>
-__global__ void __launch_bounds__(kRowThreads)
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 norm_rows_kernel(const T *__restrict__ prenorm, const T *__restrict__ norm_w, const T *__restrict__ norm_b,
                  T *__restrict__ centered, T *__restrict__ preact, T *__restrict__ predrop, T *__restrict__ out,
                  T *__restrict__ mask, T *__restrict__ rstd_out, uint32_t N, uint32_t norm, ActDrop ad,
@@ -86,9 +87,18 @@ norm_rows_kernel(const T *__restrict__ prenorm, const T *__restrict__ norm_w, co
     } else {
         mean = s / (float)N;
         float q = 0.0f;
-        for (uint32_t c = threadIdx.x; c < N; c += blockDim.x) {
-            const float d = (cached ? row_cache[c] : to_f32(prenorm[base + c])) - mean;
-            q += d * d;
+        if (vec_ok && !cached) {
+            for (uint32_t c = threadIdx.x; c < nvec; c += blockDim.x) {
+                float x[V];
+                load_run<T, V>(prenorm + base + (size_t)c * V, true, x);
+#pragma unroll
+                for (int j = 0; j < V; ++j) { const float d = x[j] - mean; q += d * d; }
+            }
+        } else {
+            for (uint32_t c = threadIdx.x; c < N; c += blockDim.x) {
+                const float d = (cached ? row_cache[c] : to_f32(prenorm[base + c])) - mean;
+                q += d * d;
+            }
         }
         q = block_sum(q, red);
         var = q / (float)N + 1e-6f;
@@ -530,6 +540,68 @@ colsum_update_kernel(const float *__restrict__ d_prenorm, const float *__restric
             for (int i = 0; i < 8; ++i) s[w] += red[w][i][cx];
         vector_step<T>(P, col, s);
     }
+}
+
+// Column sums over `M` rows of pitch `ld` and the step in one launch. A cluster owns `lanes` x V adjacent columns,
+// its blocks a contiguous share of the rows each, a thread V columns; sums are added over a block by shuffles and
+// over the cluster through distributed shared memory, in rank order, and the blocks share the columns' steps.
+// For the partial sums a dX epilogue left and for middle-sized and narrow tensors: the 10 columns of a head over 4096
+// rows take 13 us (66 us as a partial-sum launch and one that added 512 slabs one after the other), 512 x 1024 9 us
+// (13), the slabs of 1024 x 16384 9 us (11).
+template <typename T, int V>
+__global__ void __launch_bounds__(kColThreads)
+colsum_cluster_kernel(const float *__restrict__ d_prenorm, const float *__restrict__ d_norm_w,
+                     const float *__restrict__ d_norm_b, uint32_t M, uint32_t N, size_t ld, uint32_t lanes, VectorParams<T> P) {
+    __shared__ float red[3][kColThreads / 32][32];
+    __shared__ float total[3][32];
+    const uint32_t rank = tc::cluster_rank(), split = tc::cluster_size();
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t cl = threadIdx.x % lanes, rl = threadIdx.x / lanes, row_lanes = kColThreads / lanes, cols = lanes * V;
+    const uint32_t col0 = (blockIdx.x / split) * cols, col = col0 + cl * V;
+    const uint32_t r0 = (uint32_t)((uint64_t)rank * M / split), r1 = (uint32_t)((uint64_t)(rank + 1) * M / split);
+    const uint32_t sums = P.norm > 1 ? 3u : P.norm > 0 ? 2u : 1u;
+    const float *const src[3] = {d_prenorm, d_norm_w, d_norm_b};
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+        if (w >= sums) break;
+        float s[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) s[j] = 0.0f;
+        if (col < N)
+#pragma unroll 8
+            for (uint32_t r = r0 + rl; r < r1; r += row_lanes) {
+                float x[V];
+                load_run<float, V>(src[w] + r * ld + col, true, x);
+#pragma unroll
+                for (int j = 0; j < V; ++j) s[j] += x[j];
+            }
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            for (uint32_t o = 16; o >= lanes; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+            if (lane < lanes) red[w][warp][cl * V + j] = s[j];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 96) {
+        const uint32_t w = threadIdx.x / 32, c = threadIdx.x % 32;
+        if (c < cols && w < sums) {
+            float t = 0.0f;
+#pragma unroll
+            for (int i = 0; i < kColThreads / 32; ++i) t += red[w][i][c];
+            total[w][c] = t;
+        }
+    }
+    if (split > 1) tc::cluster_sync();
+    else __syncthreads();
+    if (threadIdx.x < cols && threadIdx.x % split == rank && col0 + threadIdx.x < N) {
+        float s[3] = {0.0f, 0.0f, 0.0f};
+        for (uint32_t w = 0; w < sums; ++w)
+            for (uint32_t r = 0; r < split; ++r)
+                s[w] += __uint_as_float(tc::ld_cluster_u32(tc::map_shared(tc::smem_u32(&total[w][threadIdx.x]), r)));
+        vector_step<T>(P, col0 + threadIdx.x, s);
+    }
+    __syncwarp();
+    if (split > 1) tc::cluster_sync();   // no block leaves while another still reads its sums
 }
 
 // Weight step from a finished f32 gradient (data-parallel path, after the sum over ranks).

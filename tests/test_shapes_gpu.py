@@ -30,6 +30,8 @@ CASES = [
     _spec("batchnorm_uneven_cluster", (128, 136, 10), "batch", "tanh", "f16", 1001),
     _spec("batchnorm_scalar_columns", (77, 133, 10), "batch", "tanh", "f32", 65),
     _spec("batchnorm_uncached_rows", (16, 64, 8), "batch", "sigmoid", "f32", 20011, "sgd"),
+    _spec("few_long_rows", (40, 4104, 24), "layer", "silu", "f16", 3),
+    _spec("head_over_many_rows", (48, 33, 10), "rms", "relu", "f32", 4099),
     _spec("ffma_cluster_uneven_panels", (1000, 70, 34), "layer", "silu", "f16", 33),
 ]
 
