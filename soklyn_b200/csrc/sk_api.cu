@@ -174,9 +174,9 @@ cudaError_t launch_tc_bn(sk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb
     const uint32_t sms = tc_sms(c);
     const uint32_t grid = tiles < sms ? tiles : sms;
     const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, kTcBM, BN);
-    kernel<<<grid, kTcThreads, S::kSmemBytes, c->stream>>>(ta, tb, M, N, K, idesc, group_n, epi, gate, c->tc_err, nullptr);
     c->tc_launches++;
-    return cudaGetLastError();
+    return launch_step(c->stream, sizeof(T) == 2, dim3(grid), kTcThreads, S::kSmemBytes, dim3(1), kernel, ta, tb, M, N, K, idesc, group_n, epi, gate, c->tc_err,
+                       nullptr);
 }
 
 // Tile width and cluster split of one product. Cost in microseconds of one B200 (fitted to single launches): waves
@@ -239,18 +239,8 @@ cudaError_t launch_tc_cluster(sk_ctx *c, const CUtensorMap &ta, const CUtensorMa
     }
     const uint32_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + BN - 1) / BN);
     const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, kTcBM, BN);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(tiles * split);
-    cfg.blockDim = dim3(kTcThreads);
-    cfg.dynamicSmemBytes = S::kSmemBytes;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     c->tc_launches++;
-    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, M, N, K, idesc, group_n, epi, c->tc_err);
+    return launch_step(c->stream, sizeof(T) == 2, dim3(tiles * split), kTcThreads, S::kSmemBytes, dim3(split), kernel, ta, tb, M, N, K, idesc, group_n, epi, c->tc_err);
 }
 
 // C[M x N] = A.B on the tensor cores. A_MN / B_MN: operand contiguous along M / N (else along K).
@@ -291,9 +281,8 @@ cudaError_t launch_tma_copy(sk_ctx *c, const S *src, size_t rows, size_t cols, s
     const bool vec = cols % 8 == 0 && ld * sizeof(S) % 16 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
     TmaCopyParts dst{};
     for (int i = 0; i < PARTS; ++i) dst.p[i] = parts[i];
-    tma_copy_kernel<S, PARTS><<<(unsigned)blocks, 256, 0, c->stream>>>(src, rows, (uint32_t)cols, ld, dst, vec);
     c->launches++;
-    return cudaGetLastError();
+    return launch_step(c->stream, sizeof(S) == 2, dim3((unsigned)blocks), 256, 0, dim3(1), tma_copy_kernel<S, PARTS>, src, rows, (uint32_t)cols, ld, dst, vec);
 }
 
 // Smallest shape worth the split passes, and what the split copies need of the workspace.
@@ -478,19 +467,9 @@ cudaError_t launch_norm_cols(sk_ctx *c, const sk_dense *L, uint32_t batch, const
         if (e != cudaSuccess) return e;
         attr_set[dev >> 6] |= 1ull << (dev & 63);
     }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)blocks());
-    cfg.blockDim = dim3(kRowThreads);
-    cfg.dynamicSmemBytes = cached ? bytes : 0;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, (const T *)L->prenorm, (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered,
-                              (T *)L->preact, (T *)L->predrop, (T *)L->out, (T *)L->mask, (T *)L->norm_rstd, batch, L->N, lanes,
-                              ad, cached);
+    return launch_step(c->stream, sizeof(T) == 2, dim3((unsigned)blocks()), kRowThreads, cached ? bytes : 0, dim3(split), kernel, (const T *)L->prenorm,
+                       (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered, (T *)L->preact, (T *)L->predrop, (T *)L->out,
+                       (T *)L->mask, (T *)L->norm_rstd, batch, L->N, lanes, ad, cached);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -531,12 +510,12 @@ int forward_impl(sk_ctx *c, const sk_dense *L, const void *x, uint32_t batch, ui
         const bool few = batch < (uint32_t)c->num_sms && L->N >= 4096, brief = L->N <= 1024;
         const uint32_t threads = few ? 1024 : brief ? 128 : kRowThreads;
         auto kernel = few ? norm_rows_kernel<T, 1024> : brief ? norm_rows_kernel<T, 128> : norm_rows_kernel<T, kRowThreads>;
-        kernel<<<batch, threads, use_cache ? cache_bytes : 0, c->stream>>>(
+        rc = check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3(batch), threads, use_cache ? cache_bytes : 0, dim3(1), kernel,
             (const T *)L->prenorm, (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered, (T *)L->preact,
-            (T *)L->predrop, (T *)L->out, (T *)L->mask, (T *)L->norm_rstd, L->N, L->norm, ad, vec, use_cache);
+            (T *)L->predrop, (T *)L->out, (T *)L->mask, (T *)L->norm_rstd, L->N, L->norm, ad, vec, use_cache), "forward norm");
     }
     c->launches++;
-    return check_cuda(c, cudaGetLastError(), "forward norm");
+    return rc;
 }
 
 // BatchNorm forward in phases for a batch that is split over devices (see norm_cols_phase_kernel).
@@ -573,19 +552,17 @@ int output_error_impl(sk_ctx *c, const sk_dense *L, const void *target, uint32_t
         size_t blocks = (total + kRowThreads - 1) / kRowThreads;
         const size_t cap = (size_t)c->num_sms * 16;
         if (blocks > cap) blocks = cap;
-        output_error_elem_kernel<T><<<(uint32_t)blocks, kRowThreads, 0, c->stream>>>(
-            (const T *)L->out, (const T *)L->preact, (const T *)target, master_of<T>(L->master_norm_w, L->norm_w), L->grad,
-            L->d_prenorm, L->d_norm_w, L->d_norm_b, L->dtype == SK_F32 ? nullptr : (T *)L->d_prenorm_lp,
-            (const T *)L->norm_rstd, (const T *)L->centered, (const T *)L->prenorm, rows, L->N, loss, L->norm, act, leaky);
         c->launches++;
-        return check_cuda(c, cudaGetLastError(), "output error");
+        return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((uint32_t)blocks), kRowThreads, 0, dim3(1), output_error_elem_kernel<T>,
+            (const T *)L->out, (const T *)L->preact, (const T *)target, (const float *)master_of<T>(L->master_norm_w, L->norm_w), L->grad,
+            L->d_prenorm, L->d_norm_w, L->d_norm_b, L->dtype == SK_F32 ? nullptr : (T *)L->d_prenorm_lp,
+            (const T *)L->norm_rstd, (const T *)L->centered, (const T *)L->prenorm, rows, L->N, loss, L->norm, act, leaky), "output error");
     }
-    output_error_kernel<T><<<(rows + warps - 1) / warps, kRowThreads, 0, c->stream>>>(
-        (T *)L->out, (const T *)L->preact, (const T *)target, master_of<T>(L->master_norm_w, L->norm_w), L->grad,
-        L->d_prenorm, L->d_norm_w, L->d_norm_b, L->dtype == SK_F32 ? nullptr : (T *)L->d_prenorm_lp,
-        (const T *)L->norm_rstd, (const T *)L->centered, (const T *)L->prenorm, rows, L->N, loss, L->norm, act, leaky);
     c->launches++;
-    return check_cuda(c, cudaGetLastError(), "output error");
+    return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((rows + warps - 1) / warps), kRowThreads, 0, dim3(1), output_error_kernel<T>,
+        (T *)L->out, (const T *)L->preact, (const T *)target, (const float *)master_of<T>(L->master_norm_w, L->norm_w), L->grad,
+        L->d_prenorm, L->d_norm_w, L->d_norm_b, L->dtype == SK_F32 ? nullptr : (T *)L->d_prenorm_lp,
+        (const T *)L->norm_rstd, (const T *)L->centered, (const T *)L->prenorm, rows, L->N, loss, L->norm, act, leaky), "output error");
 }
 
 template <typename T>
@@ -717,10 +694,10 @@ int column_sums_and_vector_update(sk_ctx *c, const sk_dense *L, uint32_t batch, 
     if (!handed && batch <= kSmallBatchRows) {
         c->fused_colsum_key = nullptr;
         ProfScope ps(c, SK_PROF_UPDATE);
-        colsum_update_kernel<T><<<(L->N + 31) / 32, kRowThreads, 0, c->stream>>>(L->d_prenorm, L->d_norm_w, L->d_norm_b, batch,
-                                                                             L->N, vector_params<T>(L, lin, nrm, hyp));
         c->launches++;
-        return check_cuda(c, cudaGetLastError(), "column sums + bias / norm parameter step");
+        return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((L->N + 31) / 32), kRowThreads, 0, dim3(1), colsum_update_kernel<T>, L->d_prenorm,
+                                         L->d_norm_w, L->d_norm_b, batch, L->N, vector_params<T>(L, lin, nrm, hyp)),
+                          "column sums + bias / norm parameter step");
     }
     if (handed || (uint64_t)batch * L->N <= kColsumClusterMax) {
         c->fused_colsum_key = nullptr;
@@ -737,18 +714,10 @@ int column_sums_and_vector_update(sk_ctx *c, const sk_dense *L, uint32_t batch, 
         auto blocks = [&] { return (size_t)((L->N + lanes * (vec ? 4 : 1) - 1) / (lanes * (vec ? 4 : 1))) * split; };
         // narrower column groups while the chip is not full: down to whole 32-byte sectors, or the columns there are
         while (vec ? lanes > 2 && blocks() < (size_t)c->num_sms : lanes > 8 && lanes / 2 >= L->N) lanes /= 2;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)blocks());
-        cfg.blockDim = dim3(kColThreads);
-        cfg.stream = c->stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
         c->launches++;
-        return check_cuda(c, cudaLaunchKernelEx(&cfg, vec ? colsum_cluster_kernel<T, 4> : colsum_cluster_kernel<T, 1>, p, w, b, rows,
-                                                L->N, ld, lanes, P), "column sums + bias / norm parameter step");
+    return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((unsigned)blocks()), kColThreads, 0, dim3(split),
+                                     vec ? colsum_cluster_kernel<T, 4> : colsum_cluster_kernel<T, 1>, p, w, b, rows, L->N, ld, lanes, P),
+                      "column sums + bias / norm parameter step");
     }
     int rc = SK_OK;
     uint32_t nslabs = 0;

@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <utility>
 
 namespace sk {
 
@@ -20,6 +21,39 @@ constexpr float kLossScaleInv = 1.0f / 512.0f;
 // every delta below. A power of two, so the copy loses no precision; the consumers multiply it back.
 constexpr float kLpScale = 1.0f / 16.0f;
 constexpr float kLpScaleInv = 16.0f;
+
+// ---- launches that overlap their predecessor's end ---------------------------------------
+// Kernels of the step are launched as programmatic dependents: the next kernel's blocks may be scheduled, and set up
+// barriers and tensor memory, while this one is still running. Every thread calls grid_ready() before its first
+// access to global memory, which waits until the preceding kernel has completed and its writes are visible; a chain
+// of such kernels is therefore ordered like any stream. Measured: 22 launches of a step on odd widths 184 -> 148 us,
+// 7 of a forward pass 139 -> 127, 16 recorded ones 125 -> 122. `overlap` is off for f32, whose FFMA kernels lose by
+// it (14 launches 152 -> 163 us).
+__device__ __forceinline__ void grid_ready() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_step(cudaStream_t stream, bool overlap, dim3 grid, uint32_t threads, size_t smem, dim3 cluster, void (*kernel)(P...), A &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    if (overlap) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster.x * cluster.y * cluster.z > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster.x;
+        attr[cfg.numAttrs].val.clusterDim.y = cluster.y;
+        attr[cfg.numAttrs++].val.clusterDim.z = cluster.z;
+    }
+    cfg.attrs = attr;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // ---- storage types -------------------------------------------------------------------
 __device__ __forceinline__ float to_f32(float v) { return v; }

@@ -110,6 +110,7 @@ gemm_simt_kernel(const TA *__restrict__ A, const TB *__restrict__ B, uint32_t M,
     const uint32_t split = kSplit ? gridDim.z : 1u, panels = (K + BK - 1) / BK;
     const uint32_t first = (uint32_t)((uint64_t)blockIdx.z * panels / split) * BK;
     const uint32_t end = min(K, (uint32_t)((uint64_t)(blockIdx.z + 1) * panels / split) * BK);
+    grid_ready();
     fetch(first);
     for (uint32_t k0 = first; k0 < end; k0 += BK) {
         stage();
@@ -251,6 +252,7 @@ gemm_simt128_kernel(const TA *__restrict__ A, const TB *__restrict__ B, uint32_t
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc2[i][j] = 0ull;   // two +0.0f
 
+    grid_ready();
     fetch(0);
     stage(0);
     __syncthreads();
@@ -308,31 +310,21 @@ cudaError_t launch_gemm_simt(cudaStream_t stream, int num_sms, const TA *A, size
     auto ctas = [&](uint32_t bm, uint32_t bn) { return (size_t)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
     if (ctas(128, 128) >= (size_t)num_sms) {
         dim3 grid((N + 127) / 128, (M + 127) / 128);
-        gemm_simt128_kernel<TA, TB, A_KCONTIG, B_NCONTIG, Epi>
-            <<<grid, kSimtThreads, 0, stream>>>(A, B, M, N, K, lda, ldb, a_vec, b_vec, epi);
+        return launch_step(stream, sizeof(TA) == 2, grid, kSimtThreads, 0, dim3(1), gemm_simt128_kernel<TA, TB, A_KCONTIG, B_NCONTIG, Epi>, A, B, M, N, K, lda, ldb,
+                           a_vec, b_vec, epi);
     } else if (ctas(64, 64) >= (size_t)num_sms) {
         dim3 grid((N + 63) / 64, (M + 63) / 64);
-        gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 64, 64, 4, 4, 32, Epi>
-            <<<grid, kSimtThreads, 0, stream>>>(A, B, M, N, K, lda, ldb, a_vec, b_vec, epi);
+        return launch_step(stream, sizeof(TA) == 2, grid, kSimtThreads, 0, dim3(1), gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 64, 64, 4, 4, 32, Epi>, A, B, M, N,
+                           K, lda, ldb, a_vec, b_vec, epi);
     } else {
         // a panel costs about a microsecond of round trip, a cluster's exchange about as much as two
         const uint32_t panels = (K + 63) / 64;
         uint32_t split = 1;
         for (uint32_t s = 2; sizeof(TA) == 2 && s <= 8 && s <= panels && ctas(32, 32) * s <= 4 * (size_t)num_sms; s *= 2)
             if ((panels + s - 1) / s + 2 < (split == 1 ? panels : (panels + split - 1) / split + 2)) split = s;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((N + 31) / 32, (M + 31) / 32, split);
-        cfg.blockDim = dim3(kSimtThreads);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = split;
-        cfg.attrs = attr;
-        cfg.numAttrs = split > 1 ? 1 : 0;
-        return cudaLaunchKernelEx(&cfg, gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 32, 32, 2, 2, 64, Epi>, A, B, M, N, K,
-                                  lda, ldb, a_vec, b_vec, epi);
+        return launch_step(stream, sizeof(TA) == 2, dim3((N + 31) / 32, (M + 31) / 32, split), kSimtThreads, 0, dim3(1, 1, split),
+                           gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 32, 32, 2, 2, 64, Epi>, A, B, M, N, K, lda, ldb, a_vec, b_vec, epi);
     }
-    return cudaGetLastError();
 }
 
 } // namespace sk

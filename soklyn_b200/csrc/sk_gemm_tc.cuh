@@ -152,9 +152,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const uint32_t num_kb = (K + kTcBK - 1) / kTcBK;
 
     if (warp == 0 && lane == 0) {
-        if (SPLIT) {
-            for (int i = 0; i < 3; ++i) { tc::prefetch_tensormap(&split_maps->a[i]); tc::prefetch_tensormap(&split_maps->b[i]); }
-        } else {
+        if (!SPLIT) {
             tc::prefetch_tensormap(&tmap_a);
             tc::prefetch_tensormap(&tmap_b);
         }
@@ -170,6 +168,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     __syncthreads();
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    grid_ready();
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -516,6 +515,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     __syncthreads();
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    grid_ready();
 
     if (warp == 0) {
         if (lane == 0) {

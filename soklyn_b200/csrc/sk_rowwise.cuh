@@ -62,6 +62,7 @@ norm_rows_kernel(const T *__restrict__ prenorm, const T *__restrict__ norm_w, co
     const uint32_t row = blockIdx.x;
     const size_t base = (size_t)row * N;
     const uint32_t nvec = vec_ok ? N / V : 0; // vec_ok implies N % 8 == 0
+    grid_ready();
 
     // pass 1: sum (LayerNorm) or sum of squares (RMSNorm)
     float s = 0.0f;
@@ -184,6 +185,7 @@ norm_cols_kernel(const T *__restrict__ prenorm, const T *__restrict__ norm_w, co
     const uint32_t col = (blockIdx.x / split) * cols + cl * V;
     const uint32_t r0 = (uint32_t)((uint64_t)rank * M / split), r1 = (uint32_t)((uint64_t)(rank + 1) * M / split);
     const bool live = col < N;                     // V = 8 only with N % 8 == 0
+    grid_ready();
     auto fetch = [&](uint32_t r, bool from_cache, float (&x)[V]) {
         load_run<T, V>(from_cache ? cache + (size_t)(r - r0) * cols + cl * V : prenorm + (size_t)r * N + col, true, x);
     };
@@ -324,6 +326,7 @@ output_error_kernel(T *__restrict__ out, const T *__restrict__ preact, const T *
                     uint32_t M, uint32_t N, uint32_t err_mode, uint32_t norm, uint32_t act, float leaky) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    grid_ready();
     if (row >= M) return;
     const size_t base = (size_t)row * N;
     const float inv_m = 1.0f / (float)M, inv_n = 1.0f / (float)N;
@@ -376,6 +379,7 @@ output_error_elem_kernel(const T *__restrict__ out, const T *__restrict__ preact
                          uint32_t M, uint32_t N, uint32_t err_mode, uint32_t norm, uint32_t act, float leaky) {
     constexpr int V = 8;
     const uint32_t nvec = N / V;
+    grid_ready();
     const size_t total = (size_t)M * nvec, stride = (size_t)gridDim.x * blockDim.x;
     const float inv_m = 1.0f / (float)M, inv_n = 1.0f / (float)N;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -523,6 +527,7 @@ colsum_update_kernel(const float *__restrict__ d_prenorm, const float *__restric
     const uint32_t cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
     const uint32_t col = blockIdx.x * 32 + cx;
     float sb = 0.0f, sw = 0.0f, sn = 0.0f;
+    grid_ready();
     if (col < N)
         for (uint32_t r = ry; r < M; r += 8) {
             const size_t idx = (size_t)r * N + col;
@@ -561,6 +566,7 @@ colsum_cluster_kernel(const float *__restrict__ d_prenorm, const float *__restri
     const uint32_t r0 = (uint32_t)((uint64_t)rank * M / split), r1 = (uint32_t)((uint64_t)(rank + 1) * M / split);
     const uint32_t sums = P.norm > 1 ? 3u : P.norm > 0 ? 2u : 1u;
     const float *const src[3] = {d_prenorm, d_norm_w, d_norm_b};
+    grid_ready();
 #pragma unroll
     for (int w = 0; w < 3; ++w) {
         if (w >= sums) break;
@@ -747,6 +753,7 @@ template <typename S, int PARTS>
 __global__ void __launch_bounds__(256)
 tma_copy_kernel(const S *__restrict__ src, size_t rows, uint32_t cols, size_t ld, TmaCopyParts dst, bool vec) {
     const uint32_t per_row = (cols + 7) / 8;
+    grid_ready();
     const size_t total = rows * per_row, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const size_t row = i / per_row;
