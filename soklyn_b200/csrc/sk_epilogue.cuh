@@ -185,12 +185,17 @@ template <typename T, int ACT = -1, int NORM = -1> struct EpiHidden {
 
     __device__ __forceinline__ uint32_t A() const { return ACT >= 0 ? (uint32_t)ACT : act; }
     __device__ __forceinline__ uint32_t Nm() const { return NORM >= 0 ? (uint32_t)NORM : norm; }
+    // which of the two stored activation tensors the derivative reads (the other is not fetched): the output for
+    // sigmoid, ReLU, leaky ReLU and tanh, the input for Mish, both for SiLU
+    __device__ __forceinline__ bool reads_out() const { return A() >= 1 && A() <= 6; }
+    __device__ __forceinline__ bool reads_in() const { return A() == 6 || A() == 7; }
 
     struct Pre1 { T pd, pa, mk, xv, r; };
     __device__ __forceinline__ void prefetch1(uint32_t row, uint32_t col, Pre1 &p) const {
         const size_t idx = (size_t)row * N + col;
-        p.pd = predrop[idx];
-        p.pa = preact[idx];
+        p.pd = p.pa = from_f32<T>(0.0f);
+        if (reads_out()) p.pd = predrop[idx];
+        if (reads_in()) p.pa = preact[idx];
         p.mk = mask[idx];
         if (Nm() == 1) p.xv = prenorm[idx];
         else if (Nm() >= 2) p.xv = centered[idx];
@@ -277,8 +282,8 @@ template <typename T, int ACT = -1, int NORM = -1> struct EpiHidden {
         }
         const size_t idx = (size_t)row * N + col0;
         float pd[V], pa[V], mk[V], xv[V], nw[V], rs[V];
-        load_run<T, V>(predrop + idx, true, pd);
-        load_run<T, V>(preact + idx, true, pa);
+        if (reads_out()) load_run<T, V>(predrop + idx, true, pd);
+        if (reads_in()) load_run<T, V>(preact + idx, true, pa);
         load_run<T, V>(mask + idx, true, mk);
         if (Nm() == 1) load_run<T, V>(prenorm + idx, true, xv);
         else if (Nm() >= 2) load_run<T, V>(centered + idx, true, xv);
@@ -348,8 +353,8 @@ template <typename T, int ACT = -1, int NORM = -1> struct EpiHidden {
     }
     __device__ __forceinline__ void prefetch(uint32_t row, uint32_t col0, Pre &p) const {
         const size_t idx = (size_t)row * N + col0;
-        p.pd = load_pack<T, 8>(predrop + idx);
-        p.pa = load_pack<T, 8>(preact + idx);
+        if (reads_out()) p.pd = load_pack<T, 8>(predrop + idx);
+        if (reads_in()) p.pa = load_pack<T, 8>(preact + idx);
         p.mk = load_pack<T, 8>(mask + idx);
         if (Nm() == 1) p.xv = load_pack<T, 8>(prenorm + idx);
         else if (Nm() >= 2) p.xv = load_pack<T, 8>(centered + idx);
