@@ -433,6 +433,7 @@ template <typename T, int KIND = -1, int REGU = -1> struct EpiWeightUpdate {
 
     static constexpr bool kPingPong = KIND >= 0 && REGU >= 0;
     static constexpr bool kVecOnly = kPingPong;
+    static constexpr int kGroup = kPingPong ? 2 : 1;   // 48 KB of parameters and moments in flight per SM
     struct Cols {};
     struct Pre { Pack<float, 8> p, v, m; };
     __device__ __forceinline__ void cols(uint32_t, Cols &) const {}

@@ -6,7 +6,7 @@
 // (64 deep in K) from global memory into a ring of shared-memory stages with TMA tile loads
 // (128-byte swizzle); one thread of warp 1 issues tcgen05.mma instructions (M=128, N=BN, K=16)
 // that read the stages through shared-memory descriptors and accumulate into one of two TMEM
-// accumulator buffers; eight epilogue warps drain the other buffer with tcgen05.ld, pass each
+// accumulator buffers; eight epilogue warps (4-11) drain the other buffer with tcgen05.ld, pass each
 // 32 x 32 block through shared memory so that global accesses run along rows, and apply the
 // fused epilogue functor (sk_epilogue.cuh). Mainloop and epilogue of consecutive tiles overlap.
 //
@@ -36,7 +36,11 @@ namespace sk {
 constexpr int kTcBM = 128;          // tile rows = UMMA M
 constexpr int kTcBK = 64;           // K depth of one stage: 64 x 2 B = one 128-byte swizzle row
 constexpr int kTcEpiWarps = 8;
-constexpr int kTcThreads = (2 + kTcEpiWarps) * 32;
+constexpr int kTcFirstEpi = 4;      // warps 0-3 are one warpgroup (0 loads, 1 issues MMAs, 2 and 3 have nothing to do), the epilogue two
+constexpr int kTcThreads = (kTcFirstEpi + kTcEpiWarps) * 32;
+// Registers a thread after the split between the warpgroups: 128 x 56 + 256 x 224 = 384 x 168, what the block is
+// launched with. An epilogue thread holds the loads of the next group of passes while it works on the current one.
+constexpr int kTcRegsMain = 56, kTcRegsEpi = 224;
 constexpr int kTcABytes = kTcBM * kTcBK * 2;
 constexpr uint32_t kRows1 = 4;      // rows whose loads are in flight together in an element-wise epilogue
 
@@ -172,6 +176,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
+        tc::reg_dec<kTcRegsMain>();   // in every branch: the compiler takes the smallest count that reaches a merge
         if (lane == 0) {
             uint32_t stage = 0, phase = 0, ready_chunks = 0;
             bool ok = true, gate_ok = true;
@@ -241,9 +246,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
             if (!ok) atomicCAS(err_flag, 0, gate_ok ? kTcErrProducer : kTcErrGate);
         }
-    } else if (warp == 1) {
+    } else if (warp < kTcFirstEpi) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        tc::reg_dec<kTcRegsMain>();
+        if (warp == 1 && lane == 0) {
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             // An accumulator is closed once per tile, or (SPLIT) every kSplitFlush K steps: see TcSplitMaps.
@@ -302,7 +308,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         }
     } else {
         // ---------------- epilogue ----------------
-        const uint32_t ew = warp - 2;                 // 0..7
+        tc::reg_inc<kTcRegsEpi>();
+        const uint32_t ew = warp - kTcFirstEpi;       // 0..7
         const uint32_t quarter = warp & 3;            // TMEM lanes this warp may read: 32*quarter ..
         const uint32_t half = ew >> 2;                // which half of the tile's columns
         float *buf = epi_buf + ew * (32 * 33);
@@ -560,9 +567,9 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             if (!ok) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrMma); }
             tc::umma_commit(tmem_full);
         }
-    } else {
+    } else if (warp >= kTcFirstEpi) {
         // the whole accumulator of this block to shared memory, rows that exist only
-        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t quarter = warp & 3, half = (warp - kTcFirstEpi) >> 2;
         if (!tc::mbar_wait(tmem_full, 0)) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrEpilogue); }
         tc::tc_fence_after_sync();
         if (m0 + quarter * 32 < M) {
@@ -585,13 +592,13 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     // a block whose waits ran out has filled in no valid tile: the cluster then writes nothing
     bool valid = true;
     for (uint32_t r = 0; r < split; ++r) valid = valid && tc::ld_cluster_u32(tc::map_shared(tc::smem_u32(gave_up), r)) == 0;
-    if (!VecOnly<Epi>::value && warp >= 2 && valid && !epi.vec_ok) {   // one element per lane
+    if (!VecOnly<Epi>::value && warp >= kTcFirstEpi && valid && !epi.vec_ok) {   // one element per lane
         const uint32_t rows = min((uint32_t)kTcBM, M - m0), step = kTcEpiWarps * split;
 #pragma unroll 1
         for (uint32_t c = lane; c < BN && n0 + c < N; c += 32) {
             const uint32_t base = tc::smem_u32(partial) + ((c & 4) / 4 * (BN / 2) + c / 8 * 4 + (c & 3)) * 4;
 #pragma unroll 1
-            for (uint32_t r0 = (warp - 2) * split + rank; r0 < rows; r0 += step * kRows1) {
+            for (uint32_t r0 = (warp - kTcFirstEpi) * split + rank; r0 < rows; r0 += step * kRows1) {
                 typename Epi::Pre1 p1[kRows1];
                 float v[kRows1];
 #pragma unroll
@@ -610,7 +617,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                     if (r0 + r * step < rows) epi.finish1(m0 + r0 + r * step, n0 + c, v[r], p1[r]);
             }
         }
-    } else if (warp >= 2 && valid) {
+    } else if (warp >= kTcFirstEpi && valid) {
         constexpr uint32_t kLanesRow = BN / 8, kRows = 32 / kLanesRow;      // rows per warp and pass: 1 (BN = 256) or 2
         const uint32_t units = (min((uint32_t)kTcBM, M - m0) + kRows - 1) / kRows, run = lane % kLanesRow;
         const uint32_t col = n0 + run * 8;
@@ -620,7 +627,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         typename EpiAcc<Epi>::type sums;
         if constexpr (EpiAcc<Epi>::value) epi.acc_init(sums);
 #pragma unroll 1
-        for (uint32_t u = (warp - 2) * split + rank; u < units; u += kTcEpiWarps * split) {
+        for (uint32_t u = (warp - kTcFirstEpi) * split + rank; u < units; u += kTcEpiWarps * split) {
             const uint32_t row = m0 + u * kRows + lane / kLanesRow;
             if (row >= M || col >= N) continue;
             typename Epi::Pre pre;
@@ -644,7 +651,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         // running sums: one slab per warp of the cluster, over all its rows of the tile
         if constexpr (EpiAcc<Epi>::value) {
             __syncwarp();
-            epi.slab_store(sums, (mi * split + rank) * kTcEpiWarps + warp - 2, col, kRows == 2, lane);
+            epi.slab_store(sums, (mi * split + rank) * kTcEpiWarps + warp - kTcFirstEpi, col, kRows == 2, lane);
         }
     }
     __syncwarp();

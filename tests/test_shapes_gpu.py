@@ -26,6 +26,8 @@ CASES = [
     _spec("odd_widths_copied", (333, 417, 203, 10), "layer", "mish", "f16", 301),
     _spec("odd_widths_copied_rms", (515, 266, 1001, 7), "rms", "silu", "f16", 257, dropout=0.3),
     _spec("odd_widths_persistent_tiles", (77, 2557, 130), "disabled", "sigmoid", "f16", 1950, "sgd"),
+    _spec("pairs_odd_row_tiles", (128, 2560, 136), "rms", "silu", "f16", 1900),
+    _spec("pairs_half_empty_last_pair", (72, 2824, 128), "layer", "mish", "bf16", 1801, "sgd"),
     _spec("batchnorm_five_rows", (64, 40, 16), "batch", "tanh", "f32", 5, "sgd"),
     _spec("batchnorm_uneven_cluster", (128, 136, 10), "batch", "tanh", "f16", 1001),
     _spec("batchnorm_scalar_columns", (77, 133, 10), "batch", "tanh", "f32", 65),
