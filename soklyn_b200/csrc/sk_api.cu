@@ -158,24 +158,25 @@ bool tc_eligible(const sk_ctx *c, uint32_t dtype, const void *a, size_t lda, con
 }
 
 // cudaFuncSetAttribute is per device: one bit per device ordinal and kernel instantiation.
-template <typename T, bool A_MN, bool B_MN, int BN, class Epi>
+template <typename T, bool A_MN, bool B_MN, int BN, class Epi, bool PAIR = false>
 cudaError_t launch_tc_bn(sk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb, uint32_t M, uint32_t N, uint32_t K,
                          const Epi &epi, const TcGate &gate, uint32_t group_n) {
-    using S = TcShape<BN>;
+    constexpr int smem = TcShape<PAIR ? BN / 2 : BN>::kSmemBytes;
+    constexpr uint32_t per_tile = PAIR ? 2 : 1;   // blocks that share a tile of per_tile x 128 rows
     static uint64_t attr_set[4] = {0, 0, 0, 0};   // devices 0..255
-    auto kernel = gemm_tc_kernel<A_MN, B_MN, BN, Epi>;
+    auto kernel = gemm_tc_kernel<A_MN, B_MN, BN, Epi, false, PAIR>;
     const unsigned dev = (unsigned)c->device & 255u;
     if (!(attr_set[dev >> 6] >> (dev & 63) & 1ull)) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmemBytes);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         attr_set[dev >> 6] |= 1ull << (dev & 63);
     }
-    const uint32_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + BN - 1) / BN);
-    const uint32_t sms = tc_sms(c);
-    const uint32_t grid = tiles < sms ? tiles : sms;
-    const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, kTcBM, BN);
+    const uint32_t tiles = ((M + per_tile * kTcBM - 1) / (per_tile * kTcBM)) * ((N + BN - 1) / BN);
+    const uint32_t slots = PAIR ? std::min(tc_sms(c), c->cluster_blocks[1]) / 2 : tc_sms(c);
+    const uint32_t grid = std::min(tiles, slots) * per_tile;
+    const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, per_tile * kTcBM, BN);
     c->tc_launches++;
-    return launch_step(c->stream, sizeof(T) == 2, dim3(grid), kTcThreads, S::kSmemBytes, dim3(1), kernel, ta, tb, M, N, K, idesc, group_n, epi, gate, c->tc_err,
+    return launch_step(c->stream, sizeof(T) == 2, dim3(grid), kTcThreads, smem, dim3(per_tile), kernel, ta, tb, M, N, K, idesc, group_n, epi, gate, c->tc_err,
                        nullptr);
 }
 
@@ -252,7 +253,12 @@ cudaError_t launch_gemm_tc(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, co
     const uint32_t bn = plan.bn;
     CUtensorMap ta, tb;
     const bool ok_a = A_MN ? get_tmap(c, A, dtype, M, K, lda, 64, &ta) : get_tmap(c, A, dtype, K, M, lda, kTcBM, &ta);
-    const bool ok_b = B_MN ? get_tmap(c, B, dtype, N, K, ldb, 64, &tb) : get_tmap(c, B, dtype, K, N, ldb, bn, &tb);
+    // pairs of blocks on 256 x 256 tiles, unless the rows of B arrive from other GPUs or the last row of tiles would be
+    // half empty often enough to cost more than the shared B saves
+    const uint32_t tiles_m = (M + kTcBM - 1) / kTcBM;
+    const bool pair = wide && plan.split == 1 && !gate.flags && tc_sms(c) >= 2 && c->cluster_blocks[1] >= 2 &&
+                      (tiles_m % 2 == 0 || tiles_m >= 15);
+    const bool ok_b = B_MN ? get_tmap(c, B, dtype, N, K, ldb, 64, &tb) : get_tmap(c, B, dtype, K, N, ldb, pair ? bn / 2 : bn, &tb);
     if (!ok_a || !ok_b) return cudaErrorInvalidValue;
     uint32_t group_n = c->tc_group_n;
     if (gate.flags) {   // a group of tile columns must not reach into a block of rows that arrives later
@@ -263,6 +269,7 @@ cudaError_t launch_gemm_tc(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, co
     if (plan.split > 1)
         return wide ? launch_tc_cluster<T, A_MN, B_MN, 256, Epi>(c, ta, tb, M, N, K, epi, group_n, plan.split)
                     : launch_tc_cluster<T, A_MN, B_MN, 128, Epi>(c, ta, tb, M, N, K, epi, group_n, plan.split);
+    if (pair) return launch_tc_bn<T, A_MN, B_MN, 256, Epi, true>(c, ta, tb, M, N, K, epi, gate, group_n);
     return wide ? launch_tc_bn<T, A_MN, B_MN, 256, Epi>(c, ta, tb, M, N, K, epi, gate, group_n)
                 : launch_tc_bn<T, A_MN, B_MN, 128, Epi>(c, ta, tb, M, N, K, epi, gate, group_n);
 }

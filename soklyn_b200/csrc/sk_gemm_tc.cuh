@@ -128,7 +128,13 @@ constexpr uint32_t kSplitStages = 2;
 __device__ __forceinline__ int split_a(int p) { return (0x001102 >> (4 * p)) & 0xF; }   // 2,0,1,1,0,0
 __device__ __forceinline__ int split_b(int p) { return (0x010120 >> (4 * p)) & 0xF; }   // 0,2,1,0,1,0
 
-template <bool A_MN, bool B_MN, int BN, class Epi, bool SPLIT = false>
+// PAIR kernels: the two blocks of a cluster work on one tile of 256 x 256 with tcgen05.mma.cta_group::2. Each block
+// loads its own 128 rows of A and one half of B's columns, so that B crosses from L2 to the SMs once per pair (32 KiB
+// per block and K step instead of 48: a 128 x 256 tile on one SM asks L2 for 17 TB/s at the burst rate), the stages
+// are smaller and six of them fit. The first block's producer and MMA thread lead: its full barriers count the bytes
+// of both blocks, its MMA thread issues for both, and its commits release the stages and hand over the accumulators in
+// both; each block's epilogue drains its own 128 rows and reports to the first block's tmem_empty.
+template <bool A_MN, bool B_MN, int BN, class Epi, bool SPLIT = false, bool PAIR = false>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                uint32_t M, uint32_t N, uint32_t K, uint32_t idesc, uint32_t group_n, Epi epi, TcGate gate,
@@ -139,7 +145,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     static_assert(!SPLIT || BN == 128, "SPLIT kernels use two pairs of 128-column accumulators");
     static_assert(!SPLIT || kSplitStages * kSplitStageBytes <= (uint32_t)(TcShape<BN>::kStages * TcShape<BN>::kStageBytes), "SPLIT stages fit the ring");
     constexpr uint32_t kTmemCols = kBufs * kBufCols;
-    using S = TcShape<BN>;
+    static_assert(!PAIR || (BN == 256 && !SPLIT), "pairs work on 256 x 256 tiles");
+    constexpr int kBRows = PAIR ? BN / 2 : BN;    // columns of B this block stages
+    using S = TcShape<kBRows>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *stages = smem;
@@ -151,7 +159,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + kBufs);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t tiles_m = (M + kTcBM - 1) / kTcBM, tiles_n = (N + BN - 1) / BN;
+    const uint32_t rank = PAIR ? tc::cluster_rank() : 0u;
+    constexpr uint32_t kTileM = PAIR ? 2 * kTcBM : kTcBM;
+    const uint32_t first_tile = PAIR ? blockIdx.x / 2 : blockIdx.x, step_tiles = PAIR ? gridDim.x / 2 : gridDim.x;
+    const uint32_t tiles_m = (M + kTileM - 1) / kTileM, tiles_n = (N + BN - 1) / BN;
     const uint32_t num_tiles = tiles_m * tiles_n;
     const uint32_t num_kb = (K + kTcBK - 1) / kTcBK;
 
@@ -161,15 +172,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             tc::prefetch_tensormap(&tmap_b);
         }
         for (int s = 0; s < S::kStages; ++s) { tc::mbar_init(&full_bar[s], 1); tc::mbar_init(&empty_bar[s], 1); }
-        for (uint32_t b = 0; b < kBufs; ++b) { tc::mbar_init(&tmem_full[b], 1); tc::mbar_init(&tmem_empty[b], kTcEpiWarps * 32); }
+        for (uint32_t b = 0; b < kBufs; ++b) { tc::mbar_init(&tmem_full[b], 1); tc::mbar_init(&tmem_empty[b], (PAIR ? 2 : 1) * kTcEpiWarps * 32); }
         tc::fence_barrier_init();
     }
     if (warp == 1) {
-        tc::tmem_alloc(tmem_slot, kTmemCols);
-        tc::tmem_relinquish();
+        if constexpr (PAIR) {
+            tc::tmem_alloc_pair(tmem_slot, kTmemCols);
+        } else {
+            tc::tmem_alloc(tmem_slot, kTmemCols);
+            tc::tmem_relinquish();
+        }
     }
     tc::tc_fence_before_sync();
     __syncthreads();
+    if constexpr (PAIR) tc::cluster_sync();       // the other block's barriers exist before anything arrives on them
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     grid_ready();
@@ -180,10 +196,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         if (lane == 0) {
             uint32_t stage = 0, phase = 0, ready_chunks = 0;
             bool ok = true, gate_ok = true;
-            for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+            for (uint32_t tile = first_tile; tile < num_tiles && ok; tile += step_tiles) {
                 uint32_t mi, ni;
                 tile_coords(tile, tiles_m, tiles_n, group_n, mi, ni);
-                const int32_t m0 = mi * kTcBM, n0 = ni * BN;
+                const int32_t m0 = mi * kTileM + rank * kTcBM, n0 = ni * BN;
                 if (gate.flags) {
                     // rows [n0, n0 + BN) of B: the blocks up to the one holding the tile's last row must be in
                     const uint32_t last_row = min((uint32_t)n0 + BN, N) - 1;
@@ -225,20 +241,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 } else {
                     for (uint32_t kb = 0; kb < num_kb && ok; ++kb) {
                         if (!tc::mbar_wait(&empty_bar[stage], phase ^ 1)) { ok = false; break; }
-                        tc::mbar_arrive_expect_tx(&full_bar[stage], S::kStageBytes);
+                        if (rank == 0) tc::mbar_arrive_expect_tx(&full_bar[stage], (PAIR ? 2 : 1) * S::kStageBytes);
                         uint8_t *sa = stages + stage * S::kStageBytes, *sb = sa + kTcABytes;
-                        const int32_t k0 = kb * kTcBK;
+                        const int32_t k0 = kb * kTcBK, b0 = n0 + rank * kBRows;
+                        const uint32_t lead_bar = PAIR ? tc::map_shared(tc::smem_u32(&full_bar[stage]), 0) : 0u;
+                        auto load = [&](uint8_t *to, const CUtensorMap *map, int32_t x, int32_t y) {
+                            if constexpr (PAIR) tc::tma_load_2d_pair(to, map, lead_bar, x, y);
+                            else tc::tma_load_2d(to, map, &full_bar[stage], x, y);
+                        };
                         if (A_MN) {
 #pragma unroll
-                            for (int j = 0; j < kTcBM / 64; ++j) tc::tma_load_2d(sa + j * 8192, &tmap_a, &full_bar[stage], m0 + j * 64, k0);
+                            for (int j = 0; j < kTcBM / 64; ++j) load(sa + j * 8192, &tmap_a, m0 + j * 64, k0);
                         } else {
-                            tc::tma_load_2d(sa, &tmap_a, &full_bar[stage], k0, m0);
+                            load(sa, &tmap_a, k0, m0);
                         }
                         if (B_MN) {
 #pragma unroll
-                            for (int j = 0; j < BN / 64; ++j) tc::tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[stage], n0 + j * 64, k0);
+                            for (int j = 0; j < kBRows / 64; ++j) load(sb + j * 8192, &tmap_b, b0 + j * 64, k0);
                         } else {
-                            tc::tma_load_2d(sb, &tmap_b, &full_bar[stage], k0, n0);
+                            load(sb, &tmap_b, k0, b0);
                         }
                         if (++stage == S::kStages) { stage = 0; phase ^= 1; }
                     }
@@ -249,12 +270,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     } else if (warp < kTcFirstEpi) {
         // ---------------- MMA issuer ----------------
         tc::reg_dec<kTcRegsMain>();
-        if (warp == 1 && lane == 0) {
+        if (warp == 1 && lane == 0 && rank == 0) {
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             // An accumulator is closed once per tile, or (SPLIT) every kSplitFlush K steps: see TcSplitMaps.
             const uint32_t closes = SPLIT ? (num_kb + kSplitFlush - 1) / kSplitFlush : 1u;
-            for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+            for (uint32_t tile = first_tile; tile < num_tiles && ok; tile += step_tiles) {
                 for (uint32_t cl = 0; cl < closes && ok; ++cl) {
                     if (!tc::mbar_wait(&tmem_empty[acc], acc_phase ^ 1)) { ok = false; break; }
                     tc::tc_fence_after_sync();
@@ -293,14 +314,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                                                          : tc::make_smem_desc(sa + j * 32, 16, 1024);
                                 const uint64_t db = B_MN ? tc::make_smem_desc(sb + j * 2048, 8192, 1024)
                                                          : tc::make_smem_desc(sb + j * 32, 16, 1024);
-                                tc::umma_f16(d_tmem, da, db, idesc, st > 0 || j > 0);
+                                if constexpr (PAIR) tc::umma_f16_pair(d_tmem, da, db, idesc, st > 0 || j > 0);
+                                else tc::umma_f16(d_tmem, da, db, idesc, st > 0 || j > 0);
                             }
-                            tc::umma_commit(&empty_bar[stage]);      // stage reusable once these MMAs have read it
+                            // stage reusable once these MMAs have read it
+                            if constexpr (PAIR) tc::umma_commit_pair(&empty_bar[stage]);
+                            else tc::umma_commit(&empty_bar[stage]);
                             if (++stage == S::kStages) { stage = 0; phase ^= 1; }
                         }
                     }
                     if (!ok) break;
-                    tc::umma_commit(&tmem_full[acc]);            // accumulator complete
+                    if constexpr (PAIR) tc::umma_commit_pair(&tmem_full[acc]);   // accumulator complete
+                    else tc::umma_commit(&tmem_full[acc]);
                     if (++acc == kBufs) { acc = 0; acc_phase ^= 1; }
                 }
             }
@@ -315,10 +340,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         float *buf = epi_buf + ew * (32 * 33);
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        for (uint32_t tile = first_tile; tile < num_tiles && ok; tile += step_tiles) {
             uint32_t mi, ni;
             tile_coords(tile, tiles_m, tiles_n, group_n, mi, ni);
-            const uint32_t m0 = mi * kTcBM, n0 = ni * BN;
+            const uint32_t m0 = mi * kTileM + rank * kTcBM, n0 = ni * BN;
             float part[2][32];                        // SPLIT: this thread's row, its 64 columns, summed over K
             if constexpr (SPLIT) {
 #pragma unroll
@@ -450,7 +475,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
             if constexpr (!SPLIT) {
                 tc::tc_fence_before_sync();
-                tc::mbar_arrive(&tmem_empty[acc]);
+                if constexpr (PAIR) tc::mbar_arrive_cluster(tc::map_shared(tc::smem_u32(&tmem_empty[acc]), 0));
+                else tc::mbar_arrive(&tmem_empty[acc]);
                 if (++acc == kBufs) { acc = 0; acc_phase ^= 1; }
             }
         }
@@ -459,8 +485,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
     tc::tc_fence_before_sync();
     __syncthreads();
+    if constexpr (PAIR) tc::cluster_sync();       // neither block leaves while the other's MMAs, loads or arrivals reach into it
     tc::tc_fence_after_sync();
-    if (warp == 1) tc::tmem_dealloc(tmem_base, kTmemCols);
+    if (warp == 1) {
+        if constexpr (PAIR) tc::tmem_dealloc_pair(tmem_base, kTmemCols);
+        else tc::tmem_dealloc(tmem_base, kTmemCols);
+    }
 }
 
 // ---- few output tiles: one tile per cluster, K split over its blocks ------------------------------------
