@@ -190,10 +190,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const uint32_t tmem_base = *tmem_slot;
     grid_ready();
 
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        tc::reg_dec<kTcRegsMain>();   // in every branch: the compiler takes the smallest count that reaches a merge
-        if (lane == 0) {
+    if (warp < kTcFirstEpi) {
+        tc::reg_dec<kTcRegsMain>();   // one instruction that the whole warpgroup executes, before its warps part
+        if (warp == 0 && lane == 0) {
+            // ---------------- TMA producer ----------------
             uint32_t stage = 0, phase = 0, ready_chunks = 0;
             bool ok = true, gate_ok = true;
             for (uint32_t tile = first_tile; tile < num_tiles && ok; tile += step_tiles) {
@@ -266,11 +266,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 }
             }
             if (!ok) atomicCAS(err_flag, 0, gate_ok ? kTcErrProducer : kTcErrGate);
-        }
-    } else if (warp < kTcFirstEpi) {
-        // ---------------- MMA issuer ----------------
-        tc::reg_dec<kTcRegsMain>();
-        if (warp == 1 && lane == 0 && rank == 0) {
+        } else if (warp == 1 && lane == 0 && rank == 0) {
+            // ---------------- MMA issuer ----------------
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             // An accumulator is closed once per tile, or (SPLIT) every kSplitFlush K steps: see TcSplitMaps.

@@ -1,0 +1,22 @@
+"""Rules of the kernels that the GPU does not report when they are broken, checked in the sources."""
+import os
+import re
+
+_CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "soklyn_b200", "csrc")
+
+
+def _source(name):
+    """The file without its comments."""
+    with open(os.path.join(_CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_a_warpgroup_changes_its_register_count_in_one_instruction():
+    """setmaxnreg is .aligned over the four warps of a warpgroup: they execute the same instruction, so it may stand
+    behind a condition on whole warpgroups only."""
+    users = {f: re.findall(r"tc::reg_(?:dec|inc)<", _source(f)) for f in os.listdir(_CSRC) if not f.endswith(".so")}
+    assert {f: len(u) for f, u in users.items() if u} == {"sk_gemm_tc.cuh": 2}
+    src = _source("sk_gemm_tc.cuh")
+    assert re.search(r"constexpr int kTcFirstEpi = 4;", src)
+    assert re.search(r"\n    if \(warp < kTcFirstEpi\) \{\s*tc::reg_dec<kTcRegsMain>\(\);", src)
+    assert re.search(r"\n    \} else \{\s*tc::reg_inc<kTcRegsEpi>\(\);", src)
