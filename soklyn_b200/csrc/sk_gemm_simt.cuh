@@ -154,7 +154,6 @@ gemm_simt_kernel(const TA *__restrict__ A, const TB *__restrict__ B, uint32_t M,
                 }
                 epi.template run<TN>(row, col, v, min((uint32_t)TN, N - col));
             }
-            __syncwarp();
             tc::cluster_sync();   // no block leaves while another still reads its partial tile
             return;
         }

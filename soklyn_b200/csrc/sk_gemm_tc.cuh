@@ -613,7 +613,6 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         }
         tc::tc_fence_before_sync();
     }
-    __syncwarp();
     tc::cluster_sync();
 
     // a block whose waits ran out has filled in no valid tile: the cluster then writes nothing
@@ -681,7 +680,6 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             epi.slab_store(sums, (mi * split + rank) * kTcEpiWarps + warp - kTcFirstEpi, col, kRows == 2, lane);
         }
     }
-    __syncwarp();
     tc::cluster_sync();     // no block leaves while another still reads its partial tile
     if (warp == 1) {
         tc::tc_fence_after_sync();

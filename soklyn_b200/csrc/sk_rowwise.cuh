@@ -606,7 +606,6 @@ colsum_cluster_kernel(const float *__restrict__ d_prenorm, const float *__restri
                 s[w] += __uint_as_float(tc::ld_cluster_u32(tc::map_shared(tc::smem_u32(&total[w][threadIdx.x]), r)));
         vector_step<T>(P, col0 + threadIdx.x, s);
     }
-    __syncwarp();
     if (split > 1) tc::cluster_sync();   // no block leaves while another still reads its sums
 }
 

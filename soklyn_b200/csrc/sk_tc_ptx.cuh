@@ -58,8 +58,10 @@ template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setma
 // ---- thread-block clusters ---------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
-// Every thread of every block of the cluster; shared-memory writes before it are visible cluster-wide after it.
+// Every thread of every block of the cluster; shared-memory writes before it are visible cluster-wide after it. The
+// barrier is .aligned: a warp has to arrive as one, also after a loop or branch that its lanes left at different times.
 __device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Address of this block's shared-memory word in block `rank` of the cluster, and loads through it.

@@ -20,3 +20,11 @@ def test_a_warpgroup_changes_its_register_count_in_one_instruction():
     assert re.search(r"constexpr int kTcFirstEpi = 4;", src)
     assert re.search(r"\n    if \(warp < kTcFirstEpi\) \{\s*tc::reg_dec<kTcRegsMain>\(\);", src)
     assert re.search(r"\n    \} else \{\s*tc::reg_inc<kTcRegsEpi>\(\);", src)
+
+
+def test_a_warp_arrives_at_a_cluster_barrier_as_one():
+    """barrier.cluster.*.aligned after a divergent loop is undefined: the only place that issues it brings the lanes
+    of a warp together first."""
+    uses = [(f, m.start()) for f in os.listdir(_CSRC) for m in re.finditer(r"barrier\.cluster\.arrive", _source(f))]
+    assert [f for f, _ in uses] == ["sk_tc_ptx.cuh"]
+    assert re.search(r"void cluster_sync\(\) \{\s*__syncwarp\(\);\s*asm volatile\(\"barrier\.cluster\.arrive\.release\.aligned;", _source("sk_tc_ptx.cuh"))
