@@ -149,6 +149,10 @@ inline uint32_t tc_sms(const sk_ctx *c) {
     return c->reserve_sms < n ? n - c->reserve_sms : 1u;
 }
 
+// May a launch on operands of type T overlap its predecessor's end (launch_step)? Not while SMs are reserved: the
+// blocks that wait for the predecessor would sit on the SMs it leaves free, until it ends.
+template <typename T> inline bool overlaps(const sk_ctx *c) { return sizeof(T) == 2 && c->reserve_sms == 0; }
+
 // Can the tensor-core kernel take these operands? (16-byte aligned bases, row pitches that are
 // multiples of 16 bytes, a Blackwell device, and the engine not forced to FFMA)
 bool tc_eligible(const sk_ctx *c, uint32_t dtype, const void *a, size_t lda, const void *b, size_t ldb) {
@@ -176,7 +180,7 @@ cudaError_t launch_tc_bn(sk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb
     const uint32_t grid = std::min(tiles, slots) * per_tile;
     const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, per_tile * kTcBM, BN);
     c->tc_launches++;
-    return launch_step(c->stream, sizeof(T) == 2, dim3(grid), kTcThreads, smem, dim3(per_tile), kernel, ta, tb, M, N, K, idesc, group_n, epi, gate, c->tc_err,
+    return launch_step(c->stream, overlaps<T>(c), dim3(grid), kTcThreads, smem, dim3(per_tile), kernel, ta, tb, M, N, K, idesc, group_n, epi, gate, c->tc_err,
                        nullptr);
 }
 
@@ -241,7 +245,7 @@ cudaError_t launch_tc_cluster(sk_ctx *c, const CUtensorMap &ta, const CUtensorMa
     const uint32_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + BN - 1) / BN);
     const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, kTcBM, BN);
     c->tc_launches++;
-    return launch_step(c->stream, sizeof(T) == 2, dim3(tiles * split), kTcThreads, S::kSmemBytes, dim3(split), kernel, ta, tb, M, N, K, idesc, group_n, epi, c->tc_err);
+    return launch_step(c->stream, overlaps<T>(c), dim3(tiles * split), kTcThreads, S::kSmemBytes, dim3(split), kernel, ta, tb, M, N, K, idesc, group_n, epi, c->tc_err);
 }
 
 // C[M x N] = A.B on the tensor cores. A_MN / B_MN: operand contiguous along M / N (else along K).
@@ -289,7 +293,7 @@ cudaError_t launch_tma_copy(sk_ctx *c, const S *src, size_t rows, size_t cols, s
     TmaCopyParts dst{};
     for (int i = 0; i < PARTS; ++i) dst.p[i] = parts[i];
     c->launches++;
-    return launch_step(c->stream, sizeof(S) == 2, dim3((unsigned)blocks), 256, 0, dim3(1), tma_copy_kernel<S, PARTS>, src, rows, (uint32_t)cols, ld, dst, vec);
+    return launch_step(c->stream, overlaps<S>(c), dim3((unsigned)blocks), 256, 0, dim3(1), tma_copy_kernel<S, PARTS>, src, rows, (uint32_t)cols, ld, dst, vec);
 }
 
 // Smallest shape worth the split passes, and what the split copies need of the workspace.
@@ -392,7 +396,7 @@ cudaError_t run_gemm(sk_ctx *c, uint32_t dtype, const TA *A, size_t lda, const T
         const cudaError_t e = launch_gemm_tc_split<!A_KCONTIG, B_NCONTIG, Epi>(c, A, lda, B, ldb, M, N, K, epi, &taken);
         if (taken || e != cudaSuccess) return e;
     }
-    return launch_gemm_simt<TA, TB, A_KCONTIG, B_NCONTIG, Epi>(c->stream, c->num_sms, A, lda, B, ldb, M, N, K, epi);
+    return launch_gemm_simt<TA, TB, A_KCONTIG, B_NCONTIG, Epi>(c->stream, overlaps<TA>(c), c->num_sms, A, lda, B, ldb, M, N, K, epi);
 }
 
 inline bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
@@ -474,7 +478,7 @@ cudaError_t launch_norm_cols(sk_ctx *c, const sk_dense *L, uint32_t batch, const
         if (e != cudaSuccess) return e;
         attr_set[dev >> 6] |= 1ull << (dev & 63);
     }
-    return launch_step(c->stream, sizeof(T) == 2, dim3((unsigned)blocks()), kRowThreads, cached ? bytes : 0, dim3(split), kernel, (const T *)L->prenorm,
+    return launch_step(c->stream, overlaps<T>(c), dim3((unsigned)blocks()), kRowThreads, cached ? bytes : 0, dim3(split), kernel, (const T *)L->prenorm,
                        (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered, (T *)L->preact, (T *)L->predrop, (T *)L->out,
                        (T *)L->mask, (T *)L->norm_rstd, batch, L->N, lanes, ad, cached);
 }
@@ -517,7 +521,7 @@ int forward_impl(sk_ctx *c, const sk_dense *L, const void *x, uint32_t batch, ui
         const bool few = batch < (uint32_t)c->num_sms && L->N >= 4096, brief = L->N <= 1024;
         const uint32_t threads = few ? 1024 : brief ? 128 : kRowThreads;
         auto kernel = few ? norm_rows_kernel<T, 1024> : brief ? norm_rows_kernel<T, 128> : norm_rows_kernel<T, kRowThreads>;
-        rc = check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3(batch), threads, use_cache ? cache_bytes : 0, dim3(1), kernel,
+        rc = check_cuda(c, launch_step(c->stream, overlaps<T>(c), dim3(batch), threads, use_cache ? cache_bytes : 0, dim3(1), kernel,
             (const T *)L->prenorm, (const T *)L->norm_w, (const T *)L->norm_b, (T *)L->centered, (T *)L->preact,
             (T *)L->predrop, (T *)L->out, (T *)L->mask, (T *)L->norm_rstd, L->N, L->norm, ad, vec, use_cache), "forward norm");
     }
@@ -560,13 +564,13 @@ int output_error_impl(sk_ctx *c, const sk_dense *L, const void *target, uint32_t
         const size_t cap = (size_t)c->num_sms * 16;
         if (blocks > cap) blocks = cap;
         c->launches++;
-        return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((uint32_t)blocks), kRowThreads, 0, dim3(1), output_error_elem_kernel<T>,
+        return check_cuda(c, launch_step(c->stream, overlaps<T>(c), dim3((uint32_t)blocks), kRowThreads, 0, dim3(1), output_error_elem_kernel<T>,
             (const T *)L->out, (const T *)L->preact, (const T *)target, (const float *)master_of<T>(L->master_norm_w, L->norm_w), L->grad,
             L->d_prenorm, L->d_norm_w, L->d_norm_b, L->dtype == SK_F32 ? nullptr : (T *)L->d_prenorm_lp,
             (const T *)L->norm_rstd, (const T *)L->centered, (const T *)L->prenorm, rows, L->N, loss, L->norm, act, leaky), "output error");
     }
     c->launches++;
-    return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((rows + warps - 1) / warps), kRowThreads, 0, dim3(1), output_error_kernel<T>,
+    return check_cuda(c, launch_step(c->stream, overlaps<T>(c), dim3((rows + warps - 1) / warps), kRowThreads, 0, dim3(1), output_error_kernel<T>,
         (T *)L->out, (const T *)L->preact, (const T *)target, (const float *)master_of<T>(L->master_norm_w, L->norm_w), L->grad,
         L->d_prenorm, L->d_norm_w, L->d_norm_b, L->dtype == SK_F32 ? nullptr : (T *)L->d_prenorm_lp,
         (const T *)L->norm_rstd, (const T *)L->centered, (const T *)L->prenorm, rows, L->N, loss, L->norm, act, leaky), "output error");
@@ -702,7 +706,7 @@ int column_sums_and_vector_update(sk_ctx *c, const sk_dense *L, uint32_t batch, 
         c->fused_colsum_key = nullptr;
         ProfScope ps(c, SK_PROF_UPDATE);
         c->launches++;
-        return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((L->N + 31) / 32), kRowThreads, 0, dim3(1), colsum_update_kernel<T>, L->d_prenorm,
+        return check_cuda(c, launch_step(c->stream, overlaps<T>(c), dim3((L->N + 31) / 32), kRowThreads, 0, dim3(1), colsum_update_kernel<T>, L->d_prenorm,
                                          L->d_norm_w, L->d_norm_b, batch, L->N, vector_params<T>(L, lin, nrm, hyp)),
                           "column sums + bias / norm parameter step");
     }
@@ -722,7 +726,7 @@ int column_sums_and_vector_update(sk_ctx *c, const sk_dense *L, uint32_t batch, 
         // narrower column groups while the chip is not full: down to whole 32-byte sectors, or the columns there are
         while (vec ? lanes > 2 && blocks() < (size_t)c->num_sms : lanes > 8 && lanes / 2 >= L->N) lanes /= 2;
         c->launches++;
-    return check_cuda(c, launch_step(c->stream, sizeof(T) == 2, dim3((unsigned)blocks()), kColThreads, 0, dim3(split),
+    return check_cuda(c, launch_step(c->stream, overlaps<T>(c), dim3((unsigned)blocks()), kColThreads, 0, dim3(split),
                                      vec ? colsum_cluster_kernel<T, 4> : colsum_cluster_kernel<T, 1>, p, w, b, rows, L->N, ld, lanes, P),
                       "column sums + bias / norm parameter step");
     }

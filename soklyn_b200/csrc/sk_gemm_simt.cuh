@@ -300,7 +300,7 @@ gemm_simt128_kernel(const TA *__restrict__ A, const TB *__restrict__ B, uint32_t
 
 // Host-side launcher: picks the tile so that small problems still spread over the SMs.
 template <typename TA, typename TB, bool A_KCONTIG, bool B_NCONTIG, class Epi>
-cudaError_t launch_gemm_simt(cudaStream_t stream, int num_sms, const TA *A, size_t lda, const TB *B, size_t ldb,
+cudaError_t launch_gemm_simt(cudaStream_t stream, bool overlap, int num_sms, const TA *A, size_t lda, const TB *B, size_t ldb,
                              uint32_t M, uint32_t N, uint32_t K, const Epi &epi) {
     auto aligned = [](const void *p, size_t ld, size_t es) {
         return (reinterpret_cast<uintptr_t>(p) % 16 == 0) && ((ld * es) % 16 == 0);
@@ -309,11 +309,11 @@ cudaError_t launch_gemm_simt(cudaStream_t stream, int num_sms, const TA *A, size
     auto ctas = [&](uint32_t bm, uint32_t bn) { return (size_t)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
     if (ctas(128, 128) >= (size_t)num_sms) {
         dim3 grid((N + 127) / 128, (M + 127) / 128);
-        return launch_step(stream, sizeof(TA) == 2, grid, kSimtThreads, 0, dim3(1), gemm_simt128_kernel<TA, TB, A_KCONTIG, B_NCONTIG, Epi>, A, B, M, N, K, lda, ldb,
+        return launch_step(stream, overlap, grid, kSimtThreads, 0, dim3(1), gemm_simt128_kernel<TA, TB, A_KCONTIG, B_NCONTIG, Epi>, A, B, M, N, K, lda, ldb,
                            a_vec, b_vec, epi);
     } else if (ctas(64, 64) >= (size_t)num_sms) {
         dim3 grid((N + 63) / 64, (M + 63) / 64);
-        return launch_step(stream, sizeof(TA) == 2, grid, kSimtThreads, 0, dim3(1), gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 64, 64, 4, 4, 32, Epi>, A, B, M, N,
+        return launch_step(stream, overlap, grid, kSimtThreads, 0, dim3(1), gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 64, 64, 4, 4, 32, Epi>, A, B, M, N,
                            K, lda, ldb, a_vec, b_vec, epi);
     } else {
         // a panel costs about a microsecond of round trip, a cluster's exchange about as much as two
@@ -321,7 +321,7 @@ cudaError_t launch_gemm_simt(cudaStream_t stream, int num_sms, const TA *A, size
         uint32_t split = 1;
         for (uint32_t s = 2; sizeof(TA) == 2 && s <= 8 && s <= panels && ctas(32, 32) * s <= 4 * (size_t)num_sms; s *= 2)
             if ((panels + s - 1) / s + 2 < (split == 1 ? panels : (panels + split - 1) / split + 2)) split = s;
-        return launch_step(stream, sizeof(TA) == 2, dim3((N + 31) / 32, (M + 31) / 32, split), kSimtThreads, 0, dim3(1, 1, split),
+        return launch_step(stream, overlap, dim3((N + 31) / 32, (M + 31) / 32, split), kSimtThreads, 0, dim3(1, 1, split),
                            gemm_simt_kernel<TA, TB, A_KCONTIG, B_NCONTIG, 32, 32, 2, 2, 64, Epi>, A, B, M, N, K, lda, ldb, a_vec, b_vec, epi);
     }
 }

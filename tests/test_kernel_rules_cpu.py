@@ -28,3 +28,14 @@ def test_a_warp_arrives_at_a_cluster_barrier_as_one():
     uses = [(f, m.start()) for f in os.listdir(_CSRC) for m in re.finditer(r"barrier\.cluster\.arrive", _source(f))]
     assert [f for f, _ in uses] == ["sk_tc_ptx.cuh"]
     assert re.search(r"void cluster_sync\(\) \{\s*__syncwarp\(\);\s*asm volatile\(\"barrier\.cluster\.arrive\.release\.aligned;", _source("sk_tc_ptx.cuh"))
+
+
+def test_launches_overlap_only_where_the_context_allows_it():
+    """A block that waits for the preceding kernel holds its SM, also one that SK_OPTION_RESERVE_SMS keeps free: the
+    one rule that lets a launch overlap asks for the option, and every launch of a step goes by it."""
+    api, simt = _source("sk_api.cu"), _source("sk_gemm_simt.cuh")
+    assert re.search(r"bool overlaps\(const sk_ctx \*c\) \{ return sizeof\(T\) == 2 && c->reserve_sms == 0; \}", api)
+    asks = re.findall(r"launch_step\(c->stream, (\w+)", api)
+    assert asks and set(asks) == {"overlaps"} and len(asks) == len(re.findall(r"launch_step\(", api))
+    assert set(re.findall(r"launch_step\(stream, (\w+)", simt)) == {"overlap"}
+    assert re.findall(r"launch_gemm_simt<[^;]*?>\(c->stream, (\w+)", api) == ["overlaps"]
