@@ -52,7 +52,9 @@ inline cudaError_t launch_step(cudaStream_t stream, bool overlap, dim3 grid, uin
         attr[cfg.numAttrs++].val.clusterDim.z = cluster.z;
     }
     cfg.attrs = attr;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();   // reported here: not again by the next call that asks for the last error
+    return e;
 }
 
 // ---- storage types -------------------------------------------------------------------

@@ -37,3 +37,14 @@ def test_reserved_sms_are_free_while_products_follow_each_other(gpu_ctx):
     finally:
         gpu_ctx.set_reserve_sms(0)
     assert start.elapsed_time(done) < 0.4 * start.elapsed_time(end)
+
+
+def test_a_refused_launch_is_reported_once(gpu_ctx):
+    """More rows than a grid of 128-row tiles has: the launch is refused, and the calls after it are not blamed for it."""
+    rows = 65536 * 128 + 1
+    net, x = _chain(gpu_ctx, 8, 1, rows, sk.Precision.FP32)
+    with pytest.raises(log.DriverError, match="gemm"):
+        net.forward(gpu_ctx, x, rows, False, 1)
+    assert np.all(sk.Tensor.fill(gpu_ctx, (3, 5), 2.0).download(gpu_ctx) == 2.0)
+    net.forward(gpu_ctx, x, 1000, False, 1)
+    gpu_ctx.synchronize()
