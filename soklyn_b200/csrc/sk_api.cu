@@ -615,20 +615,21 @@ int hidden_error_impl(sk_ctx *c, const sk_dense *cur, const sk_dense *next, uint
     }
     ProfScope ps(c, SK_PROF_GEMM_DX);
     cudaError_t e;
+    auto product = [&](const auto &with) { return run_gemm<T, T, true, false>(c, cur->dtype, dy, ec, wn, ec, batch, cur->N, ec, with, gate); };
     // kernels specialised for the activation / normalisation pairs of the wide and the classifier networks
-    // (they take 128-bit rows only)
-    if (!f32 && epi.vec_ok && cur->act == SK_ACT_SILU && cur->norm == SK_NORM_RMS) {
-        EpiHidden<T, SK_ACT_SILU, SK_NORM_RMS> se;
-        static_assert(sizeof(se) == sizeof(epi), "specialised functor has the same fields");
-        memcpy(&se, &epi, sizeof se);
-        e = run_gemm<T, T, true, false>(c, cur->dtype, dy, ec, wn, ec, batch, cur->N, ec, se, gate);
-    } else if (!f32 && epi.vec_ok && cur->act == SK_ACT_MISH && cur->norm == SK_NORM_LAYER) {
-        EpiHidden<T, SK_ACT_MISH, SK_NORM_LAYER> se;
-        memcpy(&se, &epi, sizeof se);
-        e = run_gemm<T, T, true, false>(c, cur->dtype, dy, ec, wn, ec, batch, cur->N, ec, se, gate);
-    } else {
-        e = run_gemm<T, T, true, false>(c, cur->dtype, dy, ec, wn, ec, batch, cur->N, ec, epi, gate);
+    // (16 bits, 128-bit rows only)
+    bool special = false;
+    if constexpr (sizeof(T) == 2) {
+        auto specialise = [&](auto se) {
+            static_assert(sizeof(se) == sizeof(epi), "specialised functor has the same fields");
+            memcpy(&se, &epi, sizeof se);
+            special = true;
+            e = product(se);
+        };
+        if (epi.vec_ok && cur->act == SK_ACT_SILU && cur->norm == SK_NORM_RMS) specialise(EpiHidden<T, SK_ACT_SILU, SK_NORM_RMS>{});
+        else if (epi.vec_ok && cur->act == SK_ACT_MISH && cur->norm == SK_NORM_LAYER) specialise(EpiHidden<T, SK_ACT_MISH, SK_NORM_LAYER>{});
     }
+    if (!special) e = product(epi);
     int rc = check_cuda(c, e, "hidden error gemm");
     if (rc) c->fused_colsum_key = nullptr;
     c->launches++;
@@ -726,9 +727,9 @@ int column_sums_and_vector_update(sk_ctx *c, const sk_dense *L, uint32_t batch, 
         // narrower column groups while the chip is not full: down to whole 32-byte sectors, or the columns there are
         while (vec ? lanes > 2 && blocks() < (size_t)c->num_sms : lanes > 8 && lanes / 2 >= L->N) lanes /= 2;
         c->launches++;
-    return check_cuda(c, launch_step(c->stream, overlaps<T>(c), dim3((unsigned)blocks()), kColThreads, 0, dim3(split),
-                                     vec ? colsum_cluster_kernel<T, 4> : colsum_cluster_kernel<T, 1>, p, w, b, rows, L->N, ld, lanes, P),
-                      "column sums + bias / norm parameter step");
+        return check_cuda(c, launch_step(c->stream, overlaps<T>(c), dim3((unsigned)blocks()), kColThreads, 0, dim3(split),
+                                         vec ? colsum_cluster_kernel<T, 4> : colsum_cluster_kernel<T, 1>, p, w, b, rows, L->N, ld, lanes, P),
+                          "column sums + bias / norm parameter step");
     }
     int rc = SK_OK;
     uint32_t nslabs = 0;
@@ -751,19 +752,19 @@ int backward_update_impl(sk_ctx *c, const sk_dense *L, const void *x, uint32_t b
     epi.gscale = f32 ? kLossScaleInv : kLossScaleInv * kLpScaleInv;
     epi.vec_ok = L->N % 8 == 0 && aligned16(L->w) && aligned16(epi.master) && aligned16(L->dv_w) && aligned16(L->dm_w);
     ProfScope ps(c, SK_PROF_GEMM_DW);
-    if (f32) {
-        rc = check_cuda(c, run_gemm<T, float, false, true>(c, L->dtype, (const T *)x, L->K, L->d_prenorm,
-                                                                    L->N, L->K, L->N, batch, epi), "weight gradient gemm");
+    auto product = [&](const auto &dy, const auto &with) {
+        using TB = std::remove_cv_t<std::remove_pointer_t<std::decay_t<decltype(dy)>>>;
+        return check_cuda(c, run_gemm<T, TB, false, true>(c, L->dtype, (const T *)x, L->K, dy, L->N, L->K, L->N, batch, with), "weight gradient gemm");
+    };
+    if constexpr (sizeof(T) == 4) {
+        rc = product((const float *)L->d_prenorm, epi);
     } else if (epi.vec_ok && lin.kind == SK_OPT_ADAM && L->regu == SK_REGU_NONE) {   // specialised: Adam, no regularisation, 128-bit rows
         EpiWeightUpdate<T, SK_OPT_ADAM, SK_REGU_NONE> se;
         static_assert(sizeof(se) == sizeof(epi), "specialised functor has the same fields");
         memcpy(&se, &epi, sizeof se);
-        rc = check_cuda(c, run_gemm<T, T, false, true>(c, L->dtype, (const T *)x, L->K, (const T *)L->d_prenorm_lp, L->N,
-                                                        L->K, L->N, batch, se), "weight gradient gemm");
+        rc = product((const T *)L->d_prenorm_lp, se);
     } else {
-        rc = check_cuda(c, run_gemm<T, T, false, true>(c, L->dtype, (const T *)x, L->K,
-                                                                (const T *)L->d_prenorm_lp, L->N, L->K, L->N, batch, epi),
-                        "weight gradient gemm");
+        rc = product((const T *)L->d_prenorm_lp, epi);
     }
     c->launches++;
     return rc;
