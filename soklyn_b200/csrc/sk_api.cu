@@ -230,22 +230,23 @@ void query_cluster_blocks(sk_ctx *c) {
     }
 }
 
-template <typename T, bool A_MN, bool B_MN, int BN, class Epi>
+template <typename T, bool A_MN, bool B_MN, int BN, class Epi, bool SUMS = false>
 cudaError_t launch_tc_cluster(sk_ctx *c, const CUtensorMap &ta, const CUtensorMap &tb, uint32_t M, uint32_t N, uint32_t K,
                               const Epi &epi, uint32_t group_n, uint32_t split) {
-    using S = TcClusterShape<BN>;
+    constexpr int smem = TcClusterShape<BN, SUMS>::kSmemBytes;
     static uint64_t attr_set[4] = {0, 0, 0, 0};   // devices 0..255
-    auto kernel = gemm_tc_cluster_kernel<A_MN, B_MN, BN, Epi>;
+    auto kernel = gemm_tc_cluster_kernel<A_MN, B_MN, BN, Epi, SUMS>;
     const unsigned dev = (unsigned)c->device & 255u;
     if (!(attr_set[dev >> 6] >> (dev & 63) & 1ull)) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmemBytes);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         attr_set[dev >> 6] |= 1ull << (dev & 63);
     }
     const uint32_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + BN - 1) / BN);
+    const uint32_t clusters = SUMS && split == 1 ? std::min(tiles, tc_sms(c)) : tiles;   // SUMS kernels work through the tiles
     const uint32_t idesc = tc::make_instr_desc(std::is_same<T, __nv_bfloat16>::value ? 1u : 0u, A_MN, B_MN, kTcBM, BN);
     c->tc_launches++;
-    return launch_step(c->stream, overlaps<T>(c), dim3(tiles * split), kTcThreads, S::kSmemBytes, dim3(split), kernel, ta, tb, M, N, K, idesc, group_n, epi, c->tc_err);
+    return launch_step(c->stream, overlaps<T>(c), dim3(clusters * split), kTcThreads, smem, dim3(split), kernel, ta, tb, M, N, K, idesc, group_n, epi, c->tc_err);
 }
 
 // C[M x N] = A.B on the tensor cores. A_MN / B_MN: operand contiguous along M / N (else along K).
@@ -344,15 +345,20 @@ cudaError_t launch_gemm_tc_split(sk_ctx *c, const float *A, size_t lda, const fl
 }
 
 // 16-bit operands whose base or row pitch TMA cannot fetch (widths that are no multiple of 8, 10-wide heads): they
-// are copied to a fetchable pitch in the workspace first. Worth it once the FFMA kernel would take longer than the
-// copies and the fixed cost of the tensor-core kernel: measured, its small tiles run at about 8 TFLOP/s of the
-// padded tile (300 x 1001 x 777: 56 us, 8192 x 10 x 512: 25 us), a copy costs 2 us and its traffic, the
+// are copied to a fetchable pitch in the workspace first and multiplied by the kernel that adds up in registers
+// (gemm_tc_cluster_kernel, SUMS), so that these products lose nothing against the FFMA kernel they otherwise run on.
+// From kSumsMinK on its sums are the more exact ones on one-sided operands too (300 long: 0.9e-7 to 1.2e-7 against 2.5e-7);
+// 64 long they are not: what a stage's four instructions truncate (1.1e-7 to 1.5e-7) is as much as the chain of 64
+// adds loses (1.2e-7). Worth it once the FFMA kernel would take
+// longer than the copies and the fixed cost of the tensor-core kernel: measured, its small tiles run at about 8 TFLOP/s
+// of the padded tile (300 x 1001 x 777: 56 us, 8192 x 10 x 512: 25 us), a copy costs 2 us and its traffic, the
 // tensor-core kernel about 10 us.
+constexpr uint32_t kSumsMinK = 256;
 template <typename T, bool A_MN, bool B_MN, class Epi>
 cudaError_t launch_gemm_tc_copied(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, const T *B, size_t ldb, uint32_t M, uint32_t N,
                                   uint32_t K, const Epi &epi, bool *taken) {
     *taken = false;
-    if (c->gemm_engine == 1 || c->cc_major != 10 || !c->encode_tiled || !c->tc_err) return cudaSuccess;
+    if (c->gemm_engine == 1 || c->cc_major != 10 || !c->encode_tiled || !c->tc_err || K < kSumsMinK) return cudaSuccess;
     auto fetchable = [](const T *p, size_t ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 8 == 0; };
     const bool copy_a = !fetchable(A, lda), copy_b = !fetchable(B, ldb);
     const size_t rows_a = A_MN ? K : M, cols_a = A_MN ? M : K, rows_b = B_MN ? K : N, cols_b = B_MN ? N : K;
@@ -373,8 +379,17 @@ cudaError_t launch_gemm_tc_copied(sk_ctx *c, uint32_t dtype, const T *A, size_t 
         if ((e = launch_tma_copy<T, 1>(c, B, rows_b, cols_b, ldb, to)) != cudaSuccess) return e;
         B = (const T *)to[0]; ldb = tma_pitch(cols_b);
     }
+    CUtensorMap ta, tb;
+    constexpr uint32_t bn = 128;   // 64 sums per epilogue thread
+    const bool ok_a = A_MN ? get_tmap(c, A, dtype, M, K, lda, 64, &ta) : get_tmap(c, A, dtype, K, M, lda, kTcBM, &ta);
+    const bool ok_b = B_MN ? get_tmap(c, B, dtype, N, K, ldb, 64, &tb) : get_tmap(c, B, dtype, K, N, ldb, bn, &tb);
+    if (!ok_a || !ok_b) return cudaErrorInvalidValue;
     *taken = true;
-    return launch_gemm_tc<T, A_MN, B_MN, Epi>(c, dtype, A, lda, B, ldb, M, N, K, epi);
+    // as large a cluster as still fits the chip in one wave: the K loop and the element-wise epilogue of a tile are both serial
+    const uint32_t num_kb = (K + kTcBK - 1) / kTcBK, tiles = ((M + kTcBM - 1) / kTcBM) * ((N + bn - 1) / bn);
+    uint32_t split = 1;
+    for (uint32_t i = 1; i < 4 && 2 * split <= num_kb && tiles * 2 * split <= std::min(tc_sms(c), c->cluster_blocks[i]); ++i) split *= 2;
+    return launch_tc_cluster<T, A_MN, B_MN, bn, Epi, true>(c, ta, tb, M, N, K, epi, c->tc_group_n, split);
 }
 
 // Engine choice for one product of the DenseBlock path.

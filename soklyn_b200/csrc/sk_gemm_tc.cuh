@@ -501,27 +501,41 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 // two planes (the first and the second four columns of every run of 8), so that a warp's remote loads are
 // contiguous: with the two halves of a run side by side, every load touched 8 rows and half of each 32-byte piece,
 // and the exchange of 16 tiles of 128 x 256 over clusters of 8 took 30 us.
-template <int BN> struct TcClusterShape {
+//
+// SUMS kernels work on operands that are fetched through a copy (odd widths), which otherwise go to the FFMA kernel and
+// its chain of round-to-nearest adds. The tensor pipe truncates when it adds into its accumulator, so here an
+// accumulator takes one stage only (64 deep, four instructions), and the epilogue warps add the stages' sums in
+// registers, round to nearest; four accumulators let the MMA thread run ahead. Error of dW in f16 against 64 bits (2-norm,
+// 1001 x 333 over 4096 rows; all-positive operands): FFMA 9.6e-7 (9.0e-7), one accumulator over K 1.1e-6 (5.5e-6), this
+// 1.1e-7 (1.1e-7); over 65536 rows 3.8e-6 (4.5e-6), 1.9e-5 (1.0e-4), 1.5e-7 (1.5e-7). They finish element by element:
+// the weight step with the exact division and square root of the FFMA kernel. A training step of 1001-4001-2003 in f16 at
+// 8192 rows takes 13.6 ms on the FFMA kernel, 2.33 ms on this one, 1.65 ms with one accumulator over K.
+template <int BN, bool SUMS = false> struct TcClusterShape {
     using S = TcShape<BN>;
     static constexpr int kPitch = BN + 4;          // floats: rows 4 banks apart, float4 accesses conflict-free both ways
-    static constexpr int kBarBytes = (2 * S::kStages + 1) * 8 + 16;
+    static constexpr int kBufs = SUMS ? 4 : 1;     // accumulators
+    static constexpr int kBarBytes = (2 * S::kStages + 2 * kBufs) * 8 + 16;
+    static_assert(!SUMS || BN == 128, "SUMS: 64 sums per thread, four accumulators of 128 columns");
     static constexpr int kSmemBytes = 1024 + S::kStages * S::kStageBytes + kBarBytes;
     static_assert(kTcBM * kPitch * 4 <= S::kStages * S::kStageBytes, "the partial tile fits the stage ring");
 };
 
-template <bool A_MN, bool B_MN, int BN, class Epi>
+template <bool A_MN, bool B_MN, int BN, class Epi, bool SUMS = false>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        uint32_t M, uint32_t N, uint32_t K, uint32_t idesc, uint32_t group_n, Epi epi, int *err_flag) {
     using S = TcShape<BN>;
-    constexpr int kPitch = TcClusterShape<BN>::kPitch;
+    using C = TcClusterShape<BN, SUMS>;
+    constexpr int kPitch = C::kPitch;
+    constexpr uint32_t kBufs = C::kBufs;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *stages = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     float *partial = reinterpret_cast<float *>(stages);
     uint64_t *full_bar = reinterpret_cast<uint64_t *>(stages + S::kStages * S::kStageBytes);
     uint64_t *empty_bar = full_bar + S::kStages;
     uint64_t *tmem_full = empty_bar + S::kStages;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_full + 1);
+    uint64_t *tmem_empty = tmem_full + kBufs;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + kBufs);
     uint32_t *gave_up = tmem_slot + 1;             // a bounded wait of this block ran out: its partial tile is not valid
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -529,20 +543,16 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const uint32_t tiles_m = (M + kTcBM - 1) / kTcBM, tiles_n = (N + BN - 1) / BN;
     const uint32_t num_kb = (K + kTcBK - 1) / kTcBK;
     const uint32_t kb0 = rank * num_kb / split, kb1 = (rank + 1) * num_kb / split;   // host: split <= num_kb <= 2^26
-    uint32_t mi, ni;
-    tile_coords(blockIdx.x / split, tiles_m, tiles_n, group_n, mi, ni);
-    const uint32_t m0 = mi * kTcBM, n0 = ni * BN;
-
     if (warp == 0 && lane == 0) {
         tc::prefetch_tensormap(&tmap_a);
         tc::prefetch_tensormap(&tmap_b);
         for (int s = 0; s < S::kStages; ++s) { tc::mbar_init(&full_bar[s], 1); tc::mbar_init(&empty_bar[s], 1); }
-        tc::mbar_init(tmem_full, 1);
+        for (uint32_t b = 0; b < kBufs; ++b) { tc::mbar_init(&tmem_full[b], 1); tc::mbar_init(&tmem_empty[b], kTcEpiWarps * 32); }
         *gave_up = 0;
         tc::fence_barrier_init();
     }
     if (warp == 1) {
-        tc::tmem_alloc(tmem_slot, BN);
+        tc::tmem_alloc(tmem_slot, kBufs * BN);
         tc::tmem_relinquish();
     }
     tc::tc_fence_before_sync();
@@ -551,139 +561,180 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const uint32_t tmem_base = *tmem_slot;
     grid_ready();
 
-    if (warp == 0) {
-        if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
-            for (uint32_t kb = kb0; kb < kb1; ++kb) {
-                if (!tc::mbar_wait(&empty_bar[stage], phase ^ 1)) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrProducer); break; }
-                tc::mbar_arrive_expect_tx(&full_bar[stage], S::kStageBytes);
-                uint8_t *sa = stages + stage * S::kStageBytes, *sb = sa + kTcABytes;
-                const int32_t k0 = kb * kTcBK;
-                if (A_MN) {
+    bool valid;
+    uint32_t tile = blockIdx.x / split, done = 0;  // SUMS: a cluster works through several tiles; stages it has been through
+    do {
+        uint32_t mi, ni;
+        tile_coords(tile, tiles_m, tiles_n, group_n, mi, ni);
+        const uint32_t m0 = mi * kTcBM, n0 = ni * BN;
+        if (warp == 0) {
+            if (lane == 0) {
+                uint32_t stage = done % S::kStages, phase = done / S::kStages & 1;
+                for (uint32_t kb = kb0; kb < kb1; ++kb) {
+                    if (!tc::mbar_wait(&empty_bar[stage], phase ^ 1)) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrProducer); break; }
+                    tc::mbar_arrive_expect_tx(&full_bar[stage], S::kStageBytes);
+                    uint8_t *sa = stages + stage * S::kStageBytes, *sb = sa + kTcABytes;
+                    const int32_t k0 = kb * kTcBK;
+                    if (A_MN) {
 #pragma unroll
-                    for (int j = 0; j < kTcBM / 64; ++j) tc::tma_load_2d(sa + j * 8192, &tmap_a, &full_bar[stage], m0 + j * 64, k0);
-                } else {
-                    tc::tma_load_2d(sa, &tmap_a, &full_bar[stage], k0, m0);
-                }
-                if (B_MN) {
+                        for (int j = 0; j < kTcBM / 64; ++j) tc::tma_load_2d(sa + j * 8192, &tmap_a, &full_bar[stage], m0 + j * 64, k0);
+                    } else {
+                        tc::tma_load_2d(sa, &tmap_a, &full_bar[stage], k0, m0);
+                    }
+                    if (B_MN) {
 #pragma unroll
-                    for (int j = 0; j < BN / 64; ++j) tc::tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[stage], n0 + j * 64, k0);
-                } else {
-                    tc::tma_load_2d(sb, &tmap_b, &full_bar[stage], k0, n0);
+                        for (int j = 0; j < BN / 64; ++j) tc::tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[stage], n0 + j * 64, k0);
+                    } else {
+                        tc::tma_load_2d(sb, &tmap_b, &full_bar[stage], k0, n0);
+                    }
+                    if (++stage == S::kStages) { stage = 0; phase ^= 1; }
                 }
-                if (++stage == S::kStages) { stage = 0; phase ^= 1; }
             }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
-            bool ok = true;
-            for (uint32_t kb = kb0; kb < kb1; ++kb) {
-                if (!tc::mbar_wait(&full_bar[stage], phase)) { ok = false; break; }
-                tc::tc_fence_after_sync();
-                const uint32_t sa = tc::smem_u32(stages + stage * S::kStageBytes), sb = sa + kTcABytes;
+        } else if (warp == 1) {
+            if (lane == 0) {
+                uint32_t stage = done % S::kStages, phase = done / S::kStages & 1;
+                bool ok = true;
+                for (uint32_t kb = kb0; kb < kb1; ++kb) {
+                    const uint32_t at = SUMS ? done + kb - kb0 : 0u, acc = at % kBufs;
+                    if (SUMS && !tc::mbar_wait(&tmem_empty[acc], (at / kBufs & 1) ^ 1)) { ok = false; break; }
+                    if (!tc::mbar_wait(&full_bar[stage], phase)) { ok = false; break; }
+                    tc::tc_fence_after_sync();
+                    const uint32_t sa = tc::smem_u32(stages + stage * S::kStageBytes), sb = sa + kTcABytes;
 #pragma unroll
-                for (int j = 0; j < kTcBK / 16; ++j) {
-                    const uint64_t da = A_MN ? tc::make_smem_desc(sa + j * 2048, 8192, 1024) : tc::make_smem_desc(sa + j * 32, 16, 1024);
-                    const uint64_t db = B_MN ? tc::make_smem_desc(sb + j * 2048, 8192, 1024) : tc::make_smem_desc(sb + j * 32, 16, 1024);
-                    tc::umma_f16(tmem_base, da, db, idesc, kb > kb0 || j > 0);
+                    for (int j = 0; j < kTcBK / 16; ++j) {
+                        const uint64_t da = A_MN ? tc::make_smem_desc(sa + j * 2048, 8192, 1024) : tc::make_smem_desc(sa + j * 32, 16, 1024);
+                        const uint64_t db = B_MN ? tc::make_smem_desc(sb + j * 2048, 8192, 1024) : tc::make_smem_desc(sb + j * 32, 16, 1024);
+                        tc::umma_f16(tmem_base + acc * BN, da, db, idesc, (!SUMS && kb > kb0) || j > 0);
+                    }
+                    tc::umma_commit(&empty_bar[stage]);
+                    if (SUMS) tc::umma_commit(&tmem_full[acc]);
+                    if (++stage == S::kStages) { stage = 0; phase ^= 1; }
                 }
-                tc::umma_commit(&empty_bar[stage]);
-                if (++stage == S::kStages) { stage = 0; phase ^= 1; }
+                if (!ok) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrMma); }
+                if (!SUMS) tc::umma_commit(tmem_full);
             }
-            if (!ok) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrMma); }
-            tc::umma_commit(tmem_full);
-        }
-    } else if (warp >= kTcFirstEpi) {
-        // the whole accumulator of this block to shared memory, rows that exist only
-        const uint32_t quarter = warp & 3, half = (warp - kTcFirstEpi) >> 2;
-        if (!tc::mbar_wait(tmem_full, 0)) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrEpilogue); }
-        tc::tc_fence_after_sync();
-        if (m0 + quarter * 32 < M) {
+        } else if (warp >= kTcFirstEpi) {
+            // the whole accumulator of this block to shared memory, rows that exist only
+            const uint32_t quarter = warp & 3, half = (warp - kTcFirstEpi) >> 2;
             float *dst = partial + (quarter * 32 + lane) * kPitch;
-#pragma unroll 1
-            for (uint32_t c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
-                if (n0 + c0 >= N) break;
-                float v[32];
-                tc::tmem_ld_32x32(tmem_base + ((quarter * 32) << 16) + c0, v);
+            auto store = [&](uint32_t c0, const float (&v)[32]) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 4)
                     *reinterpret_cast<float4 *>(dst + (j & 4) / 4 * (BN / 2) + (c0 + j) / 8 * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            }
-        }
-        tc::tc_fence_before_sync();
-    }
-    tc::cluster_sync();
-
-    // a block whose waits ran out has filled in no valid tile: the cluster then writes nothing
-    bool valid = true;
-    for (uint32_t r = 0; r < split; ++r) valid = valid && tc::ld_cluster_u32(tc::map_shared(tc::smem_u32(gave_up), r)) == 0;
-    if (!VecOnly<Epi>::value && warp >= kTcFirstEpi && valid && !epi.vec_ok) {   // one element per lane
-        const uint32_t rows = min((uint32_t)kTcBM, M - m0), step = kTcEpiWarps * split;
-#pragma unroll 1
-        for (uint32_t c = lane; c < BN && n0 + c < N; c += 32) {
-            const uint32_t base = tc::smem_u32(partial) + ((c & 4) / 4 * (BN / 2) + c / 8 * 4 + (c & 3)) * 4;
-#pragma unroll 1
-            for (uint32_t r0 = (warp - kTcFirstEpi) * split + rank; r0 < rows; r0 += step * kRows1) {
-                typename Epi::Pre1 p1[kRows1];
-                float v[kRows1];
+            };
+            if constexpr (SUMS) {
+                float sum[2][32];                      // this thread's row, its 64 columns, summed over the stages
 #pragma unroll
-                for (uint32_t r = 0; r < kRows1; ++r) {
-                    v[r] = 0.0f;
-                    if (r0 + r * step < rows) epi.prefetch1(m0 + r0 + r * step, n0 + c, p1[r]);
+                for (int j = 0; j < 32; ++j) sum[0][j] = sum[1][j] = 0.0f;
+                bool ok = true;
+                for (uint32_t at = done; at < done + kb1 - kb0 && ok; ++at) {
+                    const uint32_t acc = at % kBufs;
+                    ok = tc::mbar_wait(&tmem_full[acc], at / kBufs & 1);
+                    if (!ok) break;
+                    tc::tc_fence_after_sync();
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float v[32];
+                        tc::tmem_ld_32x32(tmem_base + ((quarter * 32) << 16) + acc * BN + half * (BN / 2) + h * 32, v);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) sum[h][j] += v[j];
+                    }
+                    tc::tc_fence_before_sync();
+                    tc::mbar_arrive(&tmem_empty[acc]);
                 }
-                for (uint32_t s = 0; s < split; ++s) {
-                    const uint32_t from = tc::map_shared(base, s);
+                if (!ok) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrEpilogue); }
+                // every stage has been read by then: the partial tile may take the ring's place
+                if (ok && m0 + quarter * 32 < M) { store(half * (BN / 2), sum[0]); store(half * (BN / 2) + 32, sum[1]); }
+            } else {
+                if (!tc::mbar_wait(tmem_full, 0)) { *gave_up = 1; atomicCAS(err_flag, 0, kTcErrEpilogue); }
+                tc::tc_fence_after_sync();
+                if (m0 + quarter * 32 < M) {
+#pragma unroll 1
+                    for (uint32_t c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
+                        if (n0 + c0 >= N) break;
+                        float v[32];
+                        tc::tmem_ld_32x32(tmem_base + ((quarter * 32) << 16) + c0, v);
+                        store(c0, v);
+                    }
+                }
+            }
+            tc::tc_fence_before_sync();
+        }
+        tc::cluster_sync();
+
+        // a block whose waits ran out has filled in no valid tile: the cluster then writes nothing
+        valid = true;
+        for (uint32_t r = 0; r < split; ++r) valid = valid && tc::ld_cluster_u32(tc::map_shared(tc::smem_u32(gave_up), r)) == 0;
+        if ((SUMS || !VecOnly<Epi>::value) && warp >= kTcFirstEpi && valid && (SUMS || !epi.vec_ok)) {   // one element per lane
+            const uint32_t rows = min((uint32_t)kTcBM, M - m0), step = kTcEpiWarps * split;
+#pragma unroll 1
+            for (uint32_t c = lane; c < BN && n0 + c < N; c += 32) {
+                const uint32_t base = tc::smem_u32(partial) + ((c & 4) / 4 * (BN / 2) + c / 8 * 4 + (c & 3)) * 4;
+#pragma unroll 1
+                for (uint32_t r0 = (warp - kTcFirstEpi) * split + rank; r0 < rows; r0 += step * kRows1) {
+                    typename Epi::Pre1 p1[kRows1];
+                    float v[kRows1];
+#pragma unroll
+                    for (uint32_t r = 0; r < kRows1; ++r) {
+                        v[r] = 0.0f;
+                        if (r0 + r * step < rows) epi.prefetch1(m0 + r0 + r * step, n0 + c, p1[r]);
+                    }
+                    for (uint32_t s = 0; s < split; ++s) {
+                        const uint32_t from = tc::map_shared(base, s);
+#pragma unroll
+                        for (uint32_t r = 0; r < kRows1; ++r)
+                            if (r0 + r * step < rows) v[r] += __uint_as_float(tc::ld_cluster_u32(from + (r0 + r * step) * kPitch * 4));
+                    }
 #pragma unroll
                     for (uint32_t r = 0; r < kRows1; ++r)
-                        if (r0 + r * step < rows) v[r] += __uint_as_float(tc::ld_cluster_u32(from + (r0 + r * step) * kPitch * 4));
+                        if (r0 + r * step < rows) epi.finish1(m0 + r0 + r * step, n0 + c, v[r], p1[r]);
                 }
-#pragma unroll
-                for (uint32_t r = 0; r < kRows1; ++r)
-                    if (r0 + r * step < rows) epi.finish1(m0 + r0 + r * step, n0 + c, v[r], p1[r]);
             }
-        }
-    } else if (warp >= kTcFirstEpi && valid) {
-        constexpr uint32_t kLanesRow = BN / 8, kRows = 32 / kLanesRow;      // rows per warp and pass: 1 (BN = 256) or 2
-        const uint32_t units = (min((uint32_t)kTcBM, M - m0) + kRows - 1) / kRows, run = lane % kLanesRow;
-        const uint32_t col = n0 + run * 8;
-        const uint32_t base = tc::smem_u32(partial) + run * 16;
-        typename Epi::Cols cols;
-        if (col < N) epi.cols(col, cols);
-        typename EpiAcc<Epi>::type sums;
-        if constexpr (EpiAcc<Epi>::value) epi.acc_init(sums);
+        } else if (!SUMS && warp >= kTcFirstEpi && valid) {
+            constexpr uint32_t kLanesRow = BN / 8, kRows = 32 / kLanesRow;      // rows per warp and pass: 1 (BN = 256) or 2
+            const uint32_t units = (min((uint32_t)kTcBM, M - m0) + kRows - 1) / kRows, run = lane % kLanesRow;
+            const uint32_t col = n0 + run * 8;
+            const uint32_t base = tc::smem_u32(partial) + run * 16;
+            typename Epi::Cols cols;
+            if (col < N) epi.cols(col, cols);
+            typename EpiAcc<Epi>::type sums;
+            if constexpr (EpiAcc<Epi>::value) epi.acc_init(sums);
 #pragma unroll 1
-        for (uint32_t u = (warp - kTcFirstEpi) * split + rank; u < units; u += kTcEpiWarps * split) {
-            const uint32_t row = m0 + u * kRows + lane / kLanesRow;
-            if (row >= M || col >= N) continue;
-            typename Epi::Pre pre;
-            epi.prefetch(row, col, pre);
-            const uint32_t at = base + (row - m0) * kPitch * 4;
-            float v[8];
+            for (uint32_t u = (warp - kTcFirstEpi) * split + rank; u < units; u += kTcEpiWarps * split) {
+                const uint32_t row = m0 + u * kRows + lane / kLanesRow;
+                if (row >= M || col >= N) continue;
+                typename Epi::Pre pre;
+                epi.prefetch(row, col, pre);
+                const uint32_t at = base + (row - m0) * kPitch * 4;
+                float v[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = 0.0f;
-            for (uint32_t r = 0; r < split; r += 2) {          // split is a power of two
-                const uint32_t a = tc::map_shared(at, r), b = tc::map_shared(at, r + 1);
-                const float4 a0 = tc::ld_cluster_f4(a), a1 = tc::ld_cluster_f4(a + BN * 2);
-                const float4 b0 = tc::ld_cluster_f4(b), b1 = tc::ld_cluster_f4(b + BN * 2);
-                v[0] += a0.x; v[1] += a0.y; v[2] += a0.z; v[3] += a0.w;
-                v[4] += a1.x; v[5] += a1.y; v[6] += a1.z; v[7] += a1.w;
-                v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
-                v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+                for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+                for (uint32_t r = 0; r < split; r += 2) {          // split is a power of two
+                    const uint32_t a = tc::map_shared(at, r), b = tc::map_shared(at, r + 1);
+                    const float4 a0 = tc::ld_cluster_f4(a), a1 = tc::ld_cluster_f4(a + BN * 2);
+                    const float4 b0 = tc::ld_cluster_f4(b), b1 = tc::ld_cluster_f4(b + BN * 2);
+                    v[0] += a0.x; v[1] += a0.y; v[2] += a0.z; v[3] += a0.w;
+                    v[4] += a1.x; v[5] += a1.y; v[6] += a1.z; v[7] += a1.w;
+                    v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
+                    v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+                }
+                if constexpr (EpiAcc<Epi>::value) epi.finish(row, col, v, pre, cols, sums);
+                else epi.finish(row, col, v, pre, cols);
             }
-            if constexpr (EpiAcc<Epi>::value) epi.finish(row, col, v, pre, cols, sums);
-            else epi.finish(row, col, v, pre, cols);
+            // running sums: one slab per warp of the cluster, over all its rows of the tile
+            if constexpr (EpiAcc<Epi>::value) {
+                __syncwarp();
+                epi.slab_store(sums, (mi * split + rank) * kTcEpiWarps + warp - kTcFirstEpi, col, kRows == 2, lane);
+            }
         }
-        // running sums: one slab per warp of the cluster, over all its rows of the tile
-        if constexpr (EpiAcc<Epi>::value) {
-            __syncwarp();
-            epi.slab_store(sums, (mi * split + rank) * kTcEpiWarps + warp - kTcFirstEpi, col, kRows == 2, lane);
-        }
-    }
-    tc::cluster_sync();     // no block leaves while another still reads its partial tile
+        if (SUMS) tc::fence_proxy_async_all();   // the next tile's loads go where the partial tile was
+        tc::cluster_sync();     // no block leaves, or loads its next tile, while another still reads its partial tile
+        done += kb1 - kb0;
+        tile += gridDim.x / split;
+    } while (SUMS && tile < tiles_m * tiles_n && valid);
     if (warp == 1) {
         tc::tc_fence_after_sync();
-        tc::tmem_dealloc(tmem_base, BN);
+        tc::tmem_dealloc(tmem_base, kBufs * BN);
     }
 }
 
