@@ -26,8 +26,10 @@ CASES = [
     _spec("odd_widths_copied", (333, 417, 203, 10), "layer", "mish", "f16", 301),
     _spec("odd_widths_copied_rms", (515, 266, 1001, 7), "rms", "silu", "f16", 257, dropout=0.3),
     _spec("odd_widths_persistent_tiles", (77, 2557, 130), "disabled", "sigmoid", "f16", 1950, "sgd"),
-    _spec("pairs_odd_row_tiles", (128, 2560, 136), "rms", "silu", "f16", 1900),
-    _spec("pairs_half_empty_last_pair", (72, 2824, 128), "layer", "mish", "bf16", 1801, "sgd"),
+    _spec("pairs_odd_row_tiles", (1896, 2296, 136), "rms", "silu", "f16", 1900),
+    _spec("pairs_half_empty_last_pair", (72, 2296, 128), "layer", "mish", "bf16", 1801, "sgd"),
+    _spec("pairs_ten_rows_in_the_last_block", (72, 2296, 128), "rms", "silu", "f16", 1930, "sgd"),
+    _spec("pairs_element_by_element", (72, 2301, 136), "disabled", "tanh", "f16", 1900),
     _spec("batchnorm_five_rows", (64, 40, 16), "batch", "tanh", "f32", 5, "sgd"),
     _spec("batchnorm_uneven_cluster", (128, 136, 10), "batch", "tanh", "f16", 1001),
     _spec("batchnorm_scalar_columns", (77, 133, 10), "batch", "tanh", "f32", 65),
@@ -38,14 +40,33 @@ CASES = [
 ]
 
 
+def _unheld(spec):
+    """Not held to the tolerance of a gradient: with Adam dv is its square, which doubles the relative error (dm holds the
+    gradient then); with SGD dv is the gradient."""
+    return ("mask",) + (("dv_w", "dv_b", "dv_nw", "dv_nb") if spec.optimiser == "adam" else ())
+
+
+def _pairs(m, n, sms=148):
+    """Does a product of m x n outputs run on pairs of SMs? 256-wide tiles have to take at most 5/4 of the time of 128-wide
+    ones by waves, leave no cluster of two a place, and come in an even number of rows or in 15 and more."""
+    rows, tiles = -(-m // 128), lambda bn: -(-m // 128) * -(-n // bn)
+    cost = lambda bn: -(-tiles(bn) // sms) * bn
+    return n > 128 and cost(256) * 4 <= cost(128) * 5 and 2 * tiles(256) > sms and (rows % 2 == 0 or rows >= 15)
+
+
+@pytest.mark.parametrize("spec", [s for s in CASES if s.name.startswith("pairs")], ids=lambda s: s.name)
+def test_the_pair_cases_run_pairs(spec):
+    assert _pairs(spec.batch, spec.dims[1])                                        # forward and the hidden delta
+    assert spec.name != "pairs_odd_row_tiles" or _pairs(spec.dims[0], spec.dims[1])   # and the weight gradient
+
+
 @pytest.mark.parametrize("spec", CASES, ids=lambda s: s.name)
 def test_step_matches_oracle_at_the_edges(gpu_ctx, spec):
     w = configs.make_weights(spec)
     x, t, _ = configs.make_data(spec)
     onet, _ = H.run_oracle(spec, w, x, t, 1)
     dnet, _ = H.run_device(gpu_ctx, spec, w, x, t, 1)
-    H.compare_states(gpu_ctx, spec, dnet, onet, {"f32": 1e-5, "f16": 1e-2, "bf16": 4e-2}[spec.precision],
-                     skip=("mask", "dv_w", "dv_b", "dv_nw", "dv_nb"))
+    H.compare_states(gpu_ctx, spec, dnet, onet, {"f32": 1e-5, "f16": 1e-2, "bf16": 4e-2}[spec.precision], skip=_unheld(spec))
 
 
 def test_f32_tensor_core_option_takes_odd_widths(gpu_ctx):
@@ -58,4 +79,4 @@ def test_f32_tensor_core_option_takes_odd_widths(gpu_ctx):
         dnet, _ = H.run_device(gpu_ctx, spec, w, x, t, 1)
     finally:
         gpu_ctx.set_f32_tensor_cores(False)
-    H.compare_states(gpu_ctx, spec, dnet, onet, 5e-5, skip=("mask", "dv_w", "dv_b", "dv_nw", "dv_nb"))
+    H.compare_states(gpu_ctx, spec, dnet, onet, 5e-5, skip=_unheld(spec))
