@@ -90,7 +90,10 @@ typedef struct {
  * ignore it. With create_stream != 0 the context creates (and owns) a non-blocking stream,
  * as the reference's GpuContext does; otherwise calls are ordered on the cudaStream_t
  * `stream`, where NULL is the legacy default stream. workspace_bytes of scratch are
- * allocated here (0 = default 256 MiB). Two tuning values are read from the environment here: SK_TC_GROUP_N
+ * allocated here (0 = default 256 MiB). It holds partial column sums and the copies of operands that the tensor cores
+ * cannot fetch as they are (SK_OPTION_GEMM_ENGINE, SK_OPTION_F32_TENSOR_CORES say how much those take); a product
+ * whose copies do not fit runs on the FFMA kernel instead, with the same results up to rounding and several times
+ * slower. Two tuning values are read from the environment here: SK_TC_GROUP_N
  * (tile columns the tensor-core kernels walk together, default 8) and SK_HANDOVER_MIN_ROWS (rows per call from
  * which a hidden block's column sums are taken in the dX epilogue, default 512). */
 int sk_ctx_create(int device, uint32_t tile_dim, void *stream, int create_stream, size_t workspace_bytes,
@@ -98,9 +101,13 @@ int sk_ctx_create(int device, uint32_t tile_dim, void *stream, int create_stream
 void sk_ctx_destroy(sk_ctx *ctx);
 /* Replace the stream later calls are ordered on (no counterpart; the reference owns one stream). */
 int sk_ctx_set_stream(sk_ctx *ctx, void *stream);
-/* Context options (no counterpart). SK_OPTION_GEMM_ENGINE: 0 = automatic (tcgen05 tensor-core
- * kernel for 16-bit operands whose row pitches are multiples of 16 bytes, FFMA kernel
- * otherwise), 1 = FFMA kernel only.
+/* Context options (no counterpart). SK_OPTION_GEMM_ENGINE: 0 = automatic, 1 = FFMA kernel only. Automatic:
+ * 16-bit operands whose bases are 16-byte aligned and whose row pitches are multiples of 8 elements go to the
+ * tcgen05 tensor-core kernels; others too, through a copy in the workspace, where the sum is at least 256 long and
+ * that is the faster way (a copy takes rows x cols rounded up to 8 x 2 bytes, rounded up to 256, for each operand
+ * that needs one; sk_ctx_reserve); the rest runs on the FFMA kernel. How a sum over K is shared between SMs, and so
+ * the last bits of a result, depends on the sizes and on how many thread-block clusters the GPU holds at once: two
+ * GPUs of one kind with different SMs switched off can differ there. On one GPU results repeat bit for bit.
  * SK_OPTION_COLSUM_HANDOVER: 1 = sk_hidden_error may take the column sums of the layer's d_prenorm /
  * d_norm_w / d_norm_b in its GEMM epilogue and hand them, through the workspace, to the next call if
  * that call is sk_backward_update / sk_backward_grads_lp for the same layer and batch (any other call
@@ -112,14 +119,15 @@ int sk_ctx_set_stream(sk_ctx *ctx, void *stream);
  * 16-bit d_prenorm_lp. A deviation from the reference, whose getters expose those tensors
  * (src/mlp.rs:446-454): they keep stale contents. Parameters come out bit-identical. Off by default.
  * SK_OPTION_RESERVE_SMS: number of SMs the tensor-core GEMMs leave free, so that a kernel on another
- * stream can run beside them. 0 by default.
- * SK_OPTION_F32_TENSOR_CORES: 1 = f32 products large enough to pay for it (M*N*K >= 2^28, row pitches multiples
- * of 8 elements) run on the tensor cores: both operands are split into three bf16 parts (8 + 8 + 8 significant
+ * stream can run beside them. Launches do not overlap their predecessor's end meanwhile. 0 by default.
+ * SK_OPTION_F32_TENSOR_CORES: 1 = f32 products large enough to pay for it (M*N*K >= 2^28), of any row pitch,
+ * run on the tensor cores: both operands are split into three bf16 parts (8 + 8 + 8 significant
  * bits) in the workspace, the six leading partial products are multiplied on the tensor cores and summed over K
  * in registers with round-to-nearest f32 adds, because the tensor pipe truncates when it adds into its own
- * accumulator (src/cuda/kernel/math.cu:8-50 is the FFMA loop this stands in for). Needs 6 bytes of workspace per operand element (sk_ctx_reserve); a
- * product whose parts do not fit runs on the FFMA kernel. Results differ from the FFMA kernel's in the order
- * and rounding of the f32 sums: a single product by up to 3e-6 of its largest element. Off by default. */
+ * accumulator (src/cuda/kernel/math.cu:8-50 is the FFMA loop this stands in for). Needs 3 x 2 bytes of workspace per
+ * element of rows x (cols rounded up to 8) of both operands, each of the six parts rounded up to 256 bytes
+ * (sk_ctx_reserve); a product whose parts do not fit runs on the FFMA kernel. Results differ from the FFMA kernel's
+ * in the order and rounding of the f32 sums: a single product by up to 3e-6 of its largest element. Off by default. */
 enum { SK_OPTION_GEMM_ENGINE = 0, SK_OPTION_COLSUM_HANDOVER = 1, SK_OPTION_LEAN_BACKWARD = 2, SK_OPTION_RESERVE_SMS = 3,
        SK_OPTION_F32_TENSOR_CORES = 4 };
 int sk_ctx_set_option(sk_ctx *ctx, uint32_t option, uint32_t value);

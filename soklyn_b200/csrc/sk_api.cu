@@ -258,8 +258,9 @@ cudaError_t launch_gemm_tc(sk_ctx *c, uint32_t dtype, const T *A, size_t lda, co
     const uint32_t bn = plan.bn;
     CUtensorMap ta, tb;
     const bool ok_a = A_MN ? get_tmap(c, A, dtype, M, K, lda, 64, &ta) : get_tmap(c, A, dtype, K, M, lda, kTcBM, &ta);
-    // pairs of blocks on 256 x 256 tiles, unless the rows of B arrive from other GPUs or the last row of tiles would be
-    // half empty often enough to cost more than the shared B saves
+    // pairs of blocks on 256 x 256 tiles, unless the rows of B arrive from other GPUs or the half-empty last row of pairs
+    // costs more than the shared B saves. Rows x 4096 x 4096, pairs against single blocks: 9 row tiles 60 against 42 us,
+    // 11 and 13 the same (75, 76), 15 63 against 69, 17 65 against 69, 21 86 against 98, 63 236 against 259.
     const uint32_t tiles_m = (M + kTcBM - 1) / kTcBM;
     const bool pair = wide && plan.split == 1 && !gate.flags && tc_sms(c) >= 2 && c->cluster_blocks[1] >= 2 &&
                       (tiles_m % 2 == 0 || tiles_m >= 15);
@@ -418,6 +419,8 @@ inline bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 1
 constexpr uint32_t kSmallBatchRows = 256;   // up to here column sums and the vector step share one launch
 // Elements up to which a cluster per column group takes them in one launch: measured 9 against 13 us at 512 x 1024, but
 // 23 against 20 us at 4096 x 1024 and 84 against 55 us at 65536 x 1024, where the plain grid streams better.
+// The slabs of a dX epilogue go to clusters whatever their size, because two stages are three launches there (fold,
+// update and their gap): 65536 x 4096 and the output block's sums 114 against 144 us, 8192 x 16384 55 against 60.
 constexpr uint64_t kColsumClusterMax = 1u << 21;
 constexpr uint32_t kHandoverMinRows = 512;   // below this a separate column-sum pass costs as little as the heavier dX epilogue (measured: 0.4 % of a step gained at 512 rows, 1.4 % at 1024, none at 256)
 constexpr uint32_t kColsumFold = 8;   // slabs the per-32-row column sums of the dX epilogue are folded into

@@ -433,7 +433,9 @@ template <typename T, int KIND = -1, int REGU = -1> struct EpiWeightUpdate {
 
     static constexpr bool kPingPong = KIND >= 0 && REGU >= 0;
     static constexpr bool kVecOnly = kPingPong;
-    static constexpr int kGroup = kPingPong ? 2 : 1;   // 48 KB of parameters and moments in flight per SM
+    // Two passes: 48 KB of parameters and moments in flight per SM. One pass measures the same: 4096 x 16384 with Adam 486
+    // us with two and 493 with one over 1024 rows, 467 and 462 over 128.
+    static constexpr int kGroup = kPingPong ? 2 : 1;
     struct Cols {};
     struct Pre { Pack<float, 8> p, v, m; };
     __device__ __forceinline__ void cols(uint32_t, Cols &) const {}

@@ -2,7 +2,8 @@
 //
 //   C[M x N] = A . B, f16 or bf16 operands, f32 accumulation in tensor memory (TMEM).
 //
-// One persistent CTA per SM walks output tiles of 128 x BN. Warp 0 streams operand panels
+// One persistent CTA per SM walks output tiles of 128 x BN (wide outputs: pairs of SMs 256 x 256, see PAIR kernels;
+// fewer tiles than SMs, and copied operands of odd widths: see gemm_tc_cluster_kernel). Warp 0 streams operand panels
 // (64 deep in K) from global memory into a ring of shared-memory stages with TMA tile loads
 // (128-byte swizzle); one thread of warp 1 issues tcgen05.mma instructions (M=128, N=BN, K=16)
 // that read the stages through shared-memory descriptors and accumulate into one of two TMEM
@@ -130,7 +131,7 @@ __device__ __forceinline__ int split_b(int p) { return (0x010120 >> (4 * p)) & 0
 
 // PAIR kernels: the two blocks of a cluster work on one tile of 256 x 256 with tcgen05.mma.cta_group::2. Each block
 // loads its own 128 rows of A and one half of B's columns, so that B crosses from L2 to the SMs once per pair (32 KiB
-// per block and K step instead of 48: a 128 x 256 tile on one SM asks L2 for 17 TB/s at the burst rate), the stages
+// per block and K step instead of 48: a 128 x 256 tile on one SM asks L2 for 19 TB/s at the burst rate), the stages
 // are smaller and six of them fit. The first block's producer and MMA thread lead: its full barriers count the bytes
 // of both blocks, its MMA thread issues for both, and its commits release the stages and hand over the accumulators in
 // both; each block's epilogue drains its own 128 rows and reports to the first block's tmem_empty.

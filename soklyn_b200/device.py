@@ -84,11 +84,12 @@ class GpuContext:
 
     def set_f32_tensor_cores(self, on: bool):
         """Large f32 products on the tensor cores (three bf16 parts per operand, six partial products, summed
-        over K in registers); needs 6 bytes of workspace per operand element (`reserve`)."""
+        over K in registers); needs 6 bytes of workspace per element of both operands, their rows rounded up to 8
+        elements and each of the six parts to 256 bytes (`reserve`), else the product runs on the FFMA kernel."""
         self._check(self.lib.sk_ctx_set_option(self.handle, 4, int(on)))
 
     def set_reserve_sms(self, count: int):
-        """SMs the tensor-core GEMMs leave free for a kernel on another stream."""
+        """SMs the tensor-core GEMMs leave free for a kernel on another stream (launches do not overlap meanwhile)."""
         self._check(self.lib.sk_ctx_set_option(self.handle, 3, int(count)))
 
     def reserve(self, workspace_bytes: int):
